@@ -334,8 +334,7 @@ int wadg_adjoint_create(wadg_app *app, int nsteps, int every, wadg_adjoint **out
   j->nseg = (nsteps + every - 1) / every;
   j->nv = (size_t)app->K * app->Nq * app->Nf;
   j->nf = (size_t)app->K * app->NfqNf * app->Nf;
-  const double g = app->p.gamma;
-  j->phys = Phys{g, g - 1.0, 1.0 / (2.0 * (g - 1.0)), app->p.tau, std::log(g - 1.0), 1.0 / (g - 1.0)};
+  j->phys = make_phys(app->p.gamma, app->p.tau);
   const size_t nst = (size_t)5 * (size_t)(every < nsteps ? every : (nsteps > 0 ? nsteps : 1));
   const size_t nst2 = j->nseg > 1 ? nst : 0;  // the second tape only when there are two segments
   struct {

@@ -101,12 +101,17 @@ __device__ __forceinline__ void ibl_series(double isb, double fb, double F, doub
   iblb = t2 * (fma(-t, fb, -t) - F);
 }
 
+template <bool B> struct BoolTag {
+  static constexpr bool value = B;
+};
+constexpr double SMALL_U = 4e-6;
+
 // WARP = true: must be called by all 32 lanes of a converged warp; when every
 // lane has u < 1e-6 for both means (nearly equal states, e.g. the whole
 // Taylor-Green field) the series are truncated at u^2 (remainders below
 // 1e-18 relative in the means and 1e-13 in their u-derivatives, which enter
 // multiplied by f < 1e-3).  SMALL = true: the caller has established u <
-// SMALL_U (4e-6) for every pair of the warp's elements (small_pairs); the
+// SMALL_U (4e-6) for every pair of the warp's elements (state_spread); the
 // truncated series without a vote (remainders below 1e-17 in the means and
 // 2e-11 in the derivatives, which enter multiplied by f < 2e-3).
 template <int DIM, bool WARP, bool SMALL = false>
@@ -250,15 +255,15 @@ __device__ __forceinline__ double lambda_dev(const AdjNode<DIM> &s, const Phys &
 }
 
 template <int DIM>
-__device__ __forceinline__ AdjNode<DIM> adj_node(const double *q, int stride, const Phys &P) {
-  const NodeState<DIM> s = node_state<DIM>(q, stride, P);
+__device__ __forceinline__ AdjNode<DIM> adj_node(const double *q, const Phys &P) {
+  const NodeState<DIM> s = node_state<DIM>(q, P);
   AdjNode<DIM> a;
   a.rho = s.rho;
 #pragma unroll
   for (int d = 0; d < DIM; ++d) a.vel[d] = s.vel[d];
   a.beta = s.beta;
-  a.lrho = s.lrho;
-  a.lbeta = s.lbeta;
+  a.lrho = log(s.rho);
+  a.lbeta = log(s.beta);
   a.irho = rcp(s.rho);
   a.ibeta = rcp(s.beta);
   return a;
@@ -448,7 +453,7 @@ adj_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
           if (c0 + j < NT && t < G * NN) {
             const int ee = e0 + t / NN, n = t % NN;
             const int k = min(k0 + ee, K - 1);
-            const AdjNode<DIM> s = adj_node<DIM>(u[j], 1, P);
+            const AdjNode<DIM> s = adj_node<DIM>(u[j], P);
             double *st = sEl + ee * C::per_elem;
             st[0 * NN + n] = s.rho;
 #pragma unroll
@@ -538,7 +543,7 @@ adj_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
     }
 
     // the pair loops: with a vote per pair (SM = false) or, where every pair
-    // of the warp's elements is nearly equal (small_pairs), without
+    // of the warp's elements is nearly equal (state_spread), without
     auto pair_loops = [&](auto small_tag) {
     constexpr bool SM = decltype(small_tag)::value;
     // volume-volume pairs over this warp's column half
@@ -622,7 +627,11 @@ adj_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
       }
     }
     };
-    if (small_pairs<DIM, NN, L>(st, l))
+    const double spread = state_spread<NN, L>(l, [&](int n, double &r, double &b) {
+      r = st[n];
+      b = st[(DIM + 1) * NN + n];
+    });
+    if (__all_sync(0xffffffffu, spread < SMALL_U))
       pair_loops(BoolTag<true>());
     else
       pair_loops(BoolTag<false>());
@@ -694,7 +703,7 @@ adj_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
           nP[d] = 0.5 * fgP[d * NF];
         }
         const double sJM = fgM[DIM * NF], sJP = fgP[DIM * NF];
-        const AdjNode<DIM> nb = adj_node<DIM>(UP, 1, P);
+        const AdjNode<DIM> nb = adj_node<DIM>(UP, P);
         const FluxCore<DIM> core = flux_core<DIM, false>(own, nb);
         flux_rev<DIM, false>(core, own, nb, nM, cM, P, pb, nullptr);
         flux_rev<DIM, false>(core, own, nb, nP, cP, P, pb, nullptr);

@@ -103,18 +103,23 @@ stage_kernel(int K, const double *__restrict__ vgeo, const double *__restrict__ 
     if (kq < K) {
       const int n = min(K - kq, G) * NF * Nf;
       const double *src = uf + (size_t)kq * NF * Nf;
-      double *dst = v.sPre + (size_t)q * G * NF * Nf;
-      for (int t = tq; t < n; t += GT) cp_async8(dst + t, src + t);
+      if (PRE) {
+        double *dst = v.sPre + (size_t)q * G * NF * Nf;
+        for (int t = tq; t < n; t += GT) cp_async8(dst + t, src + t);
+      } else {
+        for (int t = tq * 16; t < n; t += GT * 16) prefetch_l2(src + t);
+      }
+      v.fetch_geo(K, kb, q * G, tq, GT, vgeo);
     }
     cp_async_commit();
   };
   __syncthreads();  // the tables are shared by every group
   const int nb = (K + E - 1) / E;
-  if (PRE) prefetch_group(min(blockIdx.x, nb) * E);
+  prefetch_group(blockIdx.x < nb ? blockIdx.x * E : K);
 
   for (int ib = blockIdx.x; ib < nb; ib += gridDim.x) {
     const int k0 = ib * E;
-    if (PRE) cp_async_wait_all();
+    cp_async_wait_all();
     // an update group whose elements all lie past the end has nothing to do;
     // its volume groups leave together
     if (k0 + ubase >= K) break;
@@ -124,12 +129,11 @@ stage_kernel(int K, const double *__restrict__ vgeo, const double *__restrict__ 
     const bool vact = k0 + q * G < K;
     if (vact) {
       gsync();  // the group's traces staged
-      v.template prologue_group<false, GT>(K, k0, q * G, tq, vgeo, vfgeo, uq, uf, P,
-                                           PRE ? v.sPre : nullptr);
+      v.template prologue_group<GT>(K, k0, q * G, tq, vgeo, vfgeo, uq, uf, P, PRE ? v.sPre : nullptr);
       gsync();
     }
     const int knext = ib + gridDim.x < nb ? (ib + gridDim.x) * E : K;
-    if (PRE) prefetch_group(knext);  // the next batch's traces, during the pairs
+    prefetch_group(knext);  // the next batch's traces, during the pairs
     if (vact) {
       double acc[R][Nf];
       v.group_pairs(acc, P, q * G, tq, GT, gsync);

@@ -8,21 +8,42 @@
 // (Euler3Daffine.okl:327-362 and :387-406); the flux is symmetric in its two
 // states, so the sums are the same.
 //
+// The FP64 pipe bounds these kernels (two cycles per warp instruction and SM
+// quarter; DMMA shares it: 34.5 TFLOP/s of FMAs alone, 36.7 of DMMAs alone, 32
+// to 35 of both together), so the pair loops do only what depends on both
+// nodes.  With h = u/2 per node:
+//   * un = (h_i + h_j).n.  Affine elements: volume pairs take n = G^T D_ij, so
+//     un = sum_a D^a_ij (U^a_i + U^a_j) from the nodes' contravariant velocities
+//     U = G h; volume-face pairs of one face share n, so un = h_i.n + h_f.n,
+//     the first once per row and face, the second once per face node.
+//   * sums over j instead of terms (affine): sum_j F0 (h_i + h_j) = h_i sum_j F0 + sum_j F0 h_j;
+//     sum_j pa n = G^T sum_j pa D_ij, or n sum_f pa over one face; the kinetic
+//     part of the energy flux, F0 (u_i.u_j)/2, sums to 2 h_i.(sum_j F0 h_j).
+//     The same sums serve the face rows, with i and f exchanged.
+//   * curved elements: a face node keeps n_f = sum_a nr_a G^a_f, a row
+//     n_i = sum_a nr_a G^a_i per face, and a pair's direction is their sum.
+// FP64 instructions per volume / volume-face pair (3D, nearly equal states):
+// affine 56 / 54 -> 36 / 40.  Measured (the terms pair by pair before): volume +
+// surface 0.250 -> 0.219 ms (Taylor-Green, N=3, K=24576), 0.073 -> 0.063 ms (2D
+// vortex, N=3, K=32768); volume 0.548 -> 0.330 ms (curved N=4, K=10368, where the
+// wider log-mean polynomials replace the logarithms too).
+//
 // Layout.  A group of L lanes owns one element; lane l owns the R volume rows
 // i = l + L*r (register accumulators; the padding row, if any, computes on a
 // clamped index and is never stored).  Two warps share each group of G = 32/L
-// elements (one where a half of the face nodes would be fewer than L): warp h
-// walks half of the volume columns j and its own half of the face nodes,
-// [f0_h, f0_h + n_h).  At face step s lane l takes face node
-// f = f0_h + (l + s) mod n_h, so the L lanes of a group always touch L distinct
-// face rows, and the two warps never the same one: both add their R
-// contributions to one copy of the face-row accumulators in shared memory, a
-// __syncwarp between steps ordering the read-modify-writes.  The schedule is
-// fixed, so results are deterministic (no atomics).  Warps stay converged
-// throughout so that ecflux_n_warp can vote on the log-mean branch.
+// elements (one where a half of the face nodes would be fewer than L): each
+// walks its own volume columns and its own face nodes.  The face nodes come in
+// blocks: the warp's faces one after another where a face has at least L nodes
+// (FACES), else all of the warp's face nodes as one block.  At step s of a block
+// of n nodes lane l takes node (l + s) mod n, so the L lanes of a group always
+// touch L distinct face rows, and the two warps never the same one: both add
+// their R contributions to one copy of the face-row accumulators in shared
+// memory, a __syncwarp between steps ordering the read-modify-writes.  The
+// schedule is fixed, so results are deterministic (no atomics).  Warps stay
+// converged throughout so that pair_means can vote on the log-mean branch.
 //
 // Persistent CTAs: operator tables are staged in shared memory once per CTA;
-// the face weights in a rotated layout [r][s][l] so that the lanes of a step
+// the face weights in a rotated layout [node][r][l] so that the lanes of a step
 // read consecutive words.  In the volume kernel's batch loop the warps of an
 // element group synchronise only among themselves (named barriers): a
 // group's shared memory is its own, so no group waits for another.
@@ -43,11 +64,16 @@ template <int DIM, int N, int RR = 0> struct VolTile {
   static constexpr int R = (El::Nq + L - 1) / L;
   static constexpr int G = 32 / L;  // elements per warp group
   static_assert(El::NfqNf >= L, "face schedule needs NfqNf >= L");
-  // face halves of the two warps of an element (the second may be empty)
-  static constexpr int nf0 = (El::NfqNf + 1) / 2, nf1 = El::NfqNf - nf0;
-  static constexpr int H = nf1 >= L ? 2 : 1;  // warps per element group
-  __host__ __device__ static constexpr int nf(int h) { return H == 1 ? El::NfqNf : (h ? nf1 : nf0); }
+  static constexpr int H = El::NfqNf / 2 >= L ? 2 : 1;  // warps per element group
+  static constexpr bool FACES = El::Nfq >= L;           // blocks of one face
+  // the face nodes of the two warps: whole faces where a block is one, else halves
+  static constexpr int nf0 = H == 1 ? El::NfqNf : FACES ? (El::Nfaces + 1) / 2 * El::Nfq : (El::NfqNf + 1) / 2;
+  __host__ __device__ static constexpr int nf(int h) { return h ? El::NfqNf - nf0 : nf0; }
   __host__ __device__ static constexpr int f0(int h) { return h ? nf0 : 0; }
+  // the volume columns [c0(h), c0(h + 1)): so that both warps take about as many pairs
+  static constexpr int mid = (El::Nq + El::NfqNf) / 2 - nf0;
+  static constexpr int nc0 = H == 1 ? El::Nq : mid < 0 ? 0 : mid;
+  __host__ __device__ static constexpr int c0(int h) { return h == 0 ? 0 : h == 1 ? nc0 : El::Nq; }
 };
 
 template <int DIM, int N, bool CURVED, int W, int RR = 0>
@@ -57,18 +83,33 @@ struct VolPairsCfg {
   static constexpr int H = T::H;                      // warps per element group
   static constexpr int threads = 32 * W;
   static constexpr int E = (W / H) * T::G;            // elements per batch
-  // element strides in doubles: the state stride and the face-accumulator
-  // stride are 4 mod 8, so the G groups of a warp start 8 banks apart
-  // (conflict-free broadcasts, two wavefronts for a step's consecutive face rows)
-  static constexpr int pad4of8(int x) { return ((x + 3) / 8) * 8 + 4; }   // == 4 mod 8
-  static constexpr int pad2of4(int x) { return ((x + 1) / 4) * 4 + 2; }   // == 2 mod 4
-  static constexpr int NGS = CURVED ? El::Nvgeo : 0;  // geometric factors per node
+  // one direction per block and the sums of the header comment
+  static constexpr bool SPLIT = !CURVED && T::FACES;
+  // an element's state block (doubles; [2]: double2): logarithms [2][NN] |
+  // rho/2, beta [2][NN] | h0, h1 [2][NN] | 3D: h2 (SPLIT: and h.n of a face node, U^0 of a
+  // volume node) | SPLIT: the rest of U [2][Nq], 2D: h.n of the face nodes [NF] |
+  // curved: G/2 of the volume nodes [Nvgeo][Nq], n_f of the face nodes [DIM][NF]
+  static constexpr int oA = 2 * El::NN, oB = 4 * El::NN, oC = 6 * El::NN;
+  static constexpr int oD = oC + (DIM == 3 ? (SPLIT ? 2 : 1) * El::NN : 0);
+  static constexpr int oX = oD + (SPLIT ? 2 * El::Nq : 0);
+  static constexpr int oG = oX + (SPLIT && DIM == 2 ? El::NfqNf : 0);
+  static constexpr int oN = oG + (CURVED ? El::Nvgeo * El::Nq : 0);
+  static constexpr int nS = oN + (CURVED ? DIM * El::NfqNf : 0);
+  // the element strides are 2L mod 16 (the state block, read as double2 by a
+  // quarter warp at a time) or L mod 16 (single words, by a half warp), so that
+  // neighbouring elements' lanes fall into different banks
+  static constexpr int up(int x, int m) { return x % 16 == m % 16 ? x : up(x + 1, m); }
+  static constexpr int mL = T::L < 8 ? T::L : 8;
   static constexpr int mx(int a, int b) { return a > b ? a : b; }
-  // the state block of an element is reused after the pair phase for the row
-  // buffer and the update's staging arrays (3 x Nfields x Nq)
-  static constexpr int SE = pad4of8(mx((El::NS + NGS) * El::NN, 3 * El::Nfields * El::Nq));
-  static constexpr int SA = pad4of8(El::Nfields * El::NfqNf);
-  static constexpr int SN = El::Nfaces * DIM + El::Nvgeo;
+  // the state block of an element is reused after the pair phase for the
+  // update's staging arrays (3 x Nfields x Nq)
+  static constexpr int SE = up(mx(nS, 3 * El::Nfields * El::Nq), mL < 8 ? 2 * mL : 8);
+  // face-row accumulators: SPLIT [2][NF] (sum F0, sum pa), (m0, m1), 3D (m2, E), 2D E [NF];
+  // else the Nfields rows [NF]
+  static constexpr int SA = SPLIT ? up((DIM == 3 ? 6 : 5) * El::NfqNf, mL < 8 ? 2 * mL : 8)
+                                  : up(El::Nfields * El::NfqNf, mL);
+  // per-face nJ and G (affine), and the next slice's G
+  static constexpr int SN = CURVED ? 0 : El::Nfaces * DIM + 2 * El::Nvgeo;
   static constexpr int nD = DIM * El::Nq * El::Nq;
   static constexpr int nW = T::R * El::NfqNf * T::L;
   static constexpr size_t fixed = sizeof(double) * (size_t)(nD + 2 * nW + El::Nfaces * DIM);
@@ -81,28 +122,30 @@ struct VolPairsCfg {
   static constexpr size_t smem_vol = smem + (PREFETCH ? pre : 0);
 };
 
-// Shared-memory carve-up and the two phases common to both kernels.
+// Shared-memory carve-up and the phases common to the kernels.
 template <int DIM, int N, bool CURVED, int W, int RR = 0>
 struct VolPairs {
   using El = Elem<DIM, N>;
   using T = VolTile<DIM, N, RR>;
   using C = VolPairsCfg<DIM, N, CURVED, W, RR>;
-  static constexpr int Nq = El::Nq, NF = El::NfqNf, Nfq = El::Nfq, NN = El::NN, NS = El::NS;
+  static constexpr int Nq = El::Nq, NF = El::NfqNf, Nfq = El::Nfq, NN = El::NN;
   static constexpr int Nf = El::Nfields, NG = El::Nvgeo, L = T::L, R = T::R, G = T::G, E = C::E;
   static constexpr int SE = C::SE, SA = C::SA, SN = C::SN, H = C::H;
+  static constexpr bool SPLIT = C::SPLIT, FACES = T::FACES;
+  static_assert(SE % 2 == 0 && (!SPLIT || SA % 2 == 0), "double2 blocks");
 
-  double *sD, *sW1, *sW2, *sNr, *sSt, *sAcc, *sNrm, *sPre;
+  double *sD, *sW, *sD2, *sNr, *sSt, *sAcc, *sNrm, *sPre;
   int tid, h, g, l, e;
 
   __device__ __forceinline__ VolPairs(double *smem) {
-    sD = smem;                     // Drq | Dsq | Dtq, column-major
-    sW1 = sD + C::nD;              // [h][R][n_h][L]  1/2 VqLq(i, f), 0 on padding rows
-    sW2 = sW1 + C::nW;             // [h][R][n_h][L] -1/2 VfPq(f, i), 0 on padding rows
-    sNr = sW2 + C::nW;             // reference normals [Nfaces][DIM]
-    sSt = sNr + El::Nfaces * DIM;  // [E][SE]     node states (+ geometric factors)
-    sAcc = sSt + E * SE;           // [E][SA]     face-row accumulators
-    sNrm = sAcc + E * SA;          // [E][SN]     per-face nJ (affine) + G
-    sPre = sNrm + E * SN;          // [E][Nf][NF] staged face traces (volume kernel, PREFETCH)
+    sD = smem;                          // (Drq, Dsq) [2][j][i]
+    sW = sD + 2 * Nq * Nq;              // [2][node][R][L] 1/2 VqLq(i, f), -1/2 VfPq(f, i); 0 on padding rows
+    sSt = sW + 2 * C::nW;               // [E][SE]     node states
+    sAcc = sSt + E * SE;                // [E][SA]     face-row accumulators
+    sD2 = sAcc + E * SA;                // Dtq [j][i]  (3D)
+    sNr = sD2 + (DIM - 2) * Nq * Nq;    // reference normals [Nfaces][DIM]
+    sNrm = sNr + El::Nfaces * DIM;      // [E][SN]     per-face nJ, G, the next slice's G (affine)
+    sPre = sNrm + E * SN;               // [E][Nf][NF] staged face traces (volume kernel, PREFETCH)
     tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
     h = warp % H;
@@ -111,29 +154,37 @@ struct VolPairs {
     e = (warp / H) * G + g;
   }
 
+  // the block of face nodes that node p of the order [h][..] lies in: [fb, fb + n)
+  __device__ static __forceinline__ void block_of(int p, int &fb, int &n) {
+    if (FACES) {
+      fb = p / Nfq * Nfq;
+      n = Nfq;
+    } else {
+      const int hh = H == 2 && p >= T::nf0;
+      fb = T::f0(hh);
+      n = T::nf(hh);
+    }
+  }
+
   __device__ __forceinline__ void load_tables(const double *nrJ, const double *nsJ,
                                               const double *ntJ, const double *Drq,
                                               const double *Dsq, const double *Dtq,
                                               const double *VqLq, const double *VfPq) {
     for (int t = tid; t < Nq * Nq; t += blockDim.x) {
-      sD[t] = Drq[t];
-      sD[Nq * Nq + t] = Dsq[t];
-      if (DIM == 3) sD[2 * Nq * Nq + t] = Dtq[t];
+      sD[2 * t] = Drq[t];
+      sD[2 * t + 1] = Dsq[t];
+      if (DIM == 3) sD2[t] = Dtq[t];
     }
     for (int t = tid; t < C::nW; t += blockDim.x) {
-      int hh = 0, u = t;
-      if (H == 2 && u >= R * L * T::nf(0)) {
-        hh = 1;
-        u -= R * L * T::nf(0);
-      }
-      const int n_ = T::nf(hh);
-      const int ll = u % L, s = (u / L) % n_, r = u / (L * n_);
+      const int ll = t % L, r = (t / L) % R, p = t / (L * R);
+      int fb, n;
+      block_of(p, fb, n);
       const int i = ll + L * r;
-      int ff = ll + s;
-      if (ff >= n_) ff -= n_;
-      const int f = T::f0(hh) + ff;
-      sW1[t] = i < Nq ? 0.5 * VqLq[i + f * Nq] : 0.0;
-      sW2[t] = i < Nq ? -0.5 * VfPq[f + i * NF] : 0.0;
+      int ff = ll + (p - fb);
+      if (ff >= n) ff -= n;
+      const int f = fb + ff;
+      sW[2 * t] = i < Nq ? 0.5 * VqLq[i + f * Nq] : 0.0;
+      sW[2 * t + 1] = i < Nq ? -0.5 * VfPq[f + i * NF] : 0.0;
     }
     for (int t = tid; t < El::Nfaces; t += blockDim.x) {
       sNr[t * DIM + 0] = nrJ[t * Nfq];
@@ -142,18 +193,31 @@ struct VolPairs {
     }
   }
 
+  // affine: the geometric factors (constant per element, read at node 0 as
+  // Euler3Daffine.okl:205) of the slice whose first element is k0 + e0, into the next
+  // slice's slots (asynchronous copies; the prologue reads them)
+  __device__ __forceinline__ void fetch_geo(int K, int k0, int e0, int t0, int ts,
+                                            const double *vgeo) const {
+    if (CURVED) return;
+    for (int t = t0; t < G * NG; t += ts) {
+      const int ee = e0 + t / NG, c = t % NG;
+      const int k = min(k0 + ee, K - 1);
+      cp_async8(sNrm + ee * SN + El::Nfaces * DIM + NG + c, vgeo + (size_t)k * Nq * NG + c * Nq);
+    }
+  }
+
   // Node states of one element group's batch elements [e0, e0 + G), by TS
   // threads t0, t0 + TS, ...; elements past the end replicate the last
   // element so that every lane computes on valid data.  ufs: the group's
   // face traces already staged in shared memory, or null.  The states carry
-  // no logarithms unless LOGS (fill_logs adds them where a group needs
+  // no logarithms (fill_logs adds them where a group needs
   // them).  A thread's nodes go in chunks of four whose
   // loads (global for the volume nodes) are all issued before their node
   // states are computed.  The chunks run in a loop, not unrolled: unrolled,
   // the 3D affine volume + surface kernel spilled registers (20 -> 64 bytes)
   // and lost 2 %; rolled it gains 1.8 % there, 3 % in the affine volume
   // kernel, and the same 2-7 % as unrolled in the curved and 2D kernels
-  template <bool LOGS, int TS>
+  template <int TS>
   __device__ __forceinline__ void prologue_group(int K, int k0, int e0, int t0, const double *vgeo,
                                                  const double *vfgeo, const double *uq,
                                                  const double *uf, const Phys &P,
@@ -191,37 +255,72 @@ struct VolPairs {
         if (c0 + j < NT && t < G * NN) {
           const int ee = e0 + t / NN, n = t % NN;
           const int k = min(k0 + ee, K - 1);
-          const NodeState<DIM> s = node_state<DIM, LOGS>(u[j], 1, P);
+          const NodeState<DIM> s = node_state<DIM>(u[j], P);
           double *st = sSt + ee * SE;
-          st[0 * NN + n] = s.rho;
+          double hv[DIM];
 #pragma unroll
-          for (int d = 0; d < DIM; ++d) st[(1 + d) * NN + n] = 0.5 * s.vel[d];  // stored halved
-          st[(DIM + 1) * NN + n] = s.beta;
-          if (LOGS) {
-            st[(DIM + 2) * NN + n] = s.lrho;
-            st[(DIM + 3) * NN + n] = s.lbeta;
+          for (int d = 0; d < DIM; ++d) hv[d] = 0.5 * s.vel[d];
+          ((double2 *)(st + C::oA))[n] = make_double2(0.5 * s.rho, s.beta);
+          ((double2 *)(st + C::oB))[n] = make_double2(hv[0], hv[1]);
+          if (SPLIT) {
+            // contravariant velocity (volume node) or h.n (face node; n = G^T nr of its face)
+            const double *Gk = sNrm + ee * SN + El::Nfaces * DIM + NG;
+            double U[DIM];
+#pragma unroll
+            for (int a = 0; a < DIM; ++a) {
+              U[a] = 0.0;
+#pragma unroll
+              for (int d = 0; d < DIM; ++d) U[a] = fma(Gk[a * DIM + d], hv[d], U[a]);
+            }
+            double x = U[0];
+            if (n >= Nq) {
+              const double *nr = sNr + (n - Nq) / Nfq * DIM;
+              x = 0.0;
+#pragma unroll
+              for (int a = 0; a < DIM; ++a) x = fma(nr[a], U[a], x);
+            }
+            if (DIM == 3) {
+              ((double2 *)(st + C::oC))[n] = make_double2(hv[DIM - 1], x);
+              if (n < Nq) ((double2 *)(st + C::oD))[n] = make_double2(U[1], U[DIM - 1]);
+            } else if (n < Nq) {
+              ((double2 *)(st + C::oD))[n] = make_double2(U[0], U[1]);
+            } else {
+              st[C::oX + n - Nq] = x;
+            }
+          } else if (DIM == 3) {
+            st[C::oC + n] = hv[DIM - 1];
           }
           if (CURVED) {  // geometric factors stored halved: a pair's average
                          // (G_i + G_j)/2 is then one addition, with the same bits
+            if (n < Nq) {
 #pragma unroll
-            for (int c = 0; c < NG; ++c)
-              st[(NS + c) * NN + n] = 0.5 * ((n < Nq) ? vgeo[(size_t)k * Nq * NG + c * Nq + n]
-                                                      : vfgeo[(size_t)k * NF * NG + c * NF + (n - Nq)]);
+              for (int c = 0; c < NG; ++c)
+                st[C::oG + c * Nq + n] = 0.5 * vgeo[(size_t)k * Nq * NG + c * Nq + n];
+            } else {
+              const double *gf = vfgeo + (size_t)k * NF * NG + (n - Nq);
+              const double *nr = sNr + (n - Nq) / Nfq * DIM;
+#pragma unroll
+              for (int d = 0; d < DIM; ++d) {
+                double v = 0.0;
+#pragma unroll
+                for (int a = 0; a < DIM; ++a) v = fma(gf[(a * DIM + d) * NF], nr[a], v);
+                st[C::oN + d * NF + n - Nq] = 0.5 * v;
+              }
+            }
           }
         }
       }
     }
     for (int t = t0; t < G * SA; t += TS) sAcc[e0 * SA + t] = 0.0;
     if (!CURVED) {
-      for (int t = e0 + t0; t < e0 + G; t += TS) {
-        const int k = min(k0 + t, K - 1);
-        double Gk[NG];
+      for (int t = t0; t < G * (El::Nfaces + 1); t += TS) {
+        double *nm = sNrm + (e0 + t / (El::Nfaces + 1)) * SN;
+        const int fc = t % (El::Nfaces + 1);
+        const double *Gk = nm + El::Nfaces * DIM + NG;
+        if (fc == El::Nfaces) {
 #pragma unroll
-        for (int c = 0; c < NG; ++c) Gk[c] = vgeo[(size_t)k * Nq * NG + c * Nq];  // node 0 (:205)
-        double *nm = sNrm + t * SN;
-#pragma unroll
-        for (int c = 0; c < NG; ++c) nm[El::Nfaces * DIM + c] = Gk[c];
-        for (int fc = 0; fc < El::Nfaces; ++fc)
+          for (int c = 0; c < NG; ++c) nm[El::Nfaces * DIM + c] = Gk[c];
+        } else {
 #pragma unroll
           for (int d = 0; d < DIM; ++d) {
             double v = 0.0;
@@ -229,135 +328,356 @@ struct VolPairs {
             for (int a = 0; a < DIM; ++a) v = fma(Gk[a * DIM + d], sNr[fc * DIM + a], v);
             nm[fc * DIM + d] = v;
           }
+        }
       }
     }
   }
 
-  // a node's state as the pair phase keeps it: velocity stored halved (u/2)
-  __device__ __forceinline__ NodeState<DIM> load(const double *st, int n) const {
-    NodeState<DIM> s;
-    s.rho = st[n];
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) s.vel[d] = st[(1 + d) * NN + n];
-    s.beta = st[(DIM + 1) * NN + n];
-    s.lrho = st[(DIM + 2) * NN + n];
-    s.lbeta = st[(DIM + 3) * NN + n];
+  // a node's state as the pair phase keeps it: density and velocity halved
+  struct Node {
+    double hr, b, h[DIM], x, lr, lb;
+  };
+  template <int TT>
+  __device__ __forceinline__ Node load(const double *st, int n) const {
+    Node s;
+    const double2 a = ((const double2 *)(st + C::oA))[n], b = ((const double2 *)(st + C::oB))[n];
+    s.hr = a.x;
+    s.b = a.y;
+    s.h[0] = b.x;
+    s.h[1] = b.y;
+    s.x = 0.0;
+    if (DIM == 3) {
+      if (SPLIT) {
+        const double2 c = ((const double2 *)(st + C::oC))[n];
+        s.h[DIM - 1] = c.x;
+        s.x = c.y;
+      } else {
+        s.h[DIM - 1] = st[C::oC + n];
+      }
+    }
+    s.lr = s.lb = 0.0;
+    if (TT == 3) {
+      const double2 c = ((const double2 *)st)[n];
+      s.lr = c.x;
+      s.lb = c.y;
+    }
     return s;
   }
 
-  // all flux pairs of element e: this warp's half of the volume columns and of
-  // the face nodes; rows into acc (registers), face rows into the element's
-  // face accumulators
-  // SMALL: every pair of the warp's elements has u < SMALL_U (small_pairs),
-  // so the fluxes take the u^2 series without a vote
-  template <bool SMALL>
-  __device__ __forceinline__ void pairs(double (&acc)[R][Nf], const Phys &P) const {
+  // all flux pairs of element e: this warp's volume columns and face nodes;
+  // the rows into F (registers), the face rows into the element's face
+  // accumulators (SPLIT: the sums that face_row combines).  TT: the range of
+  // the states (state_range).
+  template <int TT>
+  __device__ __forceinline__ void pairs(double (&F)[R][Nf], const Phys &P) const {
     const double *st = sSt + e * SE;
     double *acc_f = sAcc + e * SA;
-    NodeState<DIM> A[R];
+    double ahr[R], ab[R], alr[R], alb[R], ah[R][DIM];
+    double a0[R], am[R][DIM], ap[R][DIM], aE[R];  // sums of F0, F0 h_j (else Fm), pa n, FE
     int ir[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       ir[r] = min(l + L * r, Nq - 1);  // padding row computes on a clamped index
-      A[r] = load(st, ir[r]);
+      const Node s = load<TT>(st, ir[r]);
+      ahr[r] = s.hr;
+      ab[r] = s.b;
+      alr[r] = s.lr;
+      alb[r] = s.lb;
+      a0[r] = aE[r] = 0.0;
 #pragma unroll
-      for (int q = 0; q < Nf; ++q) acc[r][q] = 0.0;
+      for (int d = 0; d < DIM; ++d) {
+        ah[r][d] = s.h[d];
+        am[r][d] = ap[r][d] = 0.0;
+      }
     }
-    double Ge[NG];
-    if (!CURVED) {
-#pragma unroll
-      for (int c = 0; c < NG; ++c) Ge[c] = sNrm[e * SN + El::Nfaces * DIM + c];
-    }
+    double rl[R], pa[R], ib[R], pf[R];
 
-    // volume-volume pairs: warp h takes columns [j0, j1)
-    const int j0 = (H == 2 && h) ? Nq / 2 : 0, j1 = (H == 2 && !h) ? Nq / 2 : Nq;
-    for (int j = j0; j < j1; ++j) {
-      const NodeState<DIM> B = load(st, j);
-      double nv[R][DIM], F[R][Nf];
+    // volume-volume pairs
+    {
+      double U[R][DIM], Ge[NG];
+      if (SPLIT) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int i = ir[r];
-        double rr[DIM];
+        for (int r = 0; r < R; ++r) {
+          const double2 u = ((const double2 *)(st + C::oD))[ir[r]];
+          if (DIM == 3) U[r][0] = st[C::oC + 2 * ir[r] + 1];
+          U[r][DIM - 2] = u.x;
+          U[r][DIM - 1] = u.y;
+        }
+      } else if (!CURVED) {
 #pragma unroll
-        for (int a = 0; a < DIM; ++a) rr[a] = sD[a * Nq * Nq + i + j * Nq];
+        for (int c = 0; c < NG; ++c) Ge[c] = sNrm[e * SN + El::Nfaces * DIM + c];
+      }
+      for (int j = T::c0(h); j < T::c0(h + 1 + (H == 1)); ++j) {
+        const Node B = load<TT>(st, j);
+        double UB[DIM];
+        if (SPLIT) {
+          const double2 u = ((const double2 *)(st + C::oD))[j];
+          if (DIM == 3) UB[0] = B.x;
+          UB[DIM - 2] = u.x;
+          UB[DIM - 1] = u.y;
+        }
+        pair_means<R, TT>(ahr, ab, alr, alb, B.hr, B.b, B.lr, B.lb, P, rl, pa, ib, pf);
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) {
-          double v = 0.0;
+        for (int r = 0; r < R; ++r) {
+          double D[DIM];
+          const double2 d2 = ((const double2 *)sD)[ir[r] + j * Nq];
+          D[0] = d2.x;
+          D[1] = d2.y;
+          if (DIM == 3) D[DIM - 1] = sD2[ir[r] + j * Nq];
+          if (SPLIT) {
+            double un = 0.0;
 #pragma unroll
-          for (int a = 0; a < DIM; ++a) {
-            const double gad = CURVED ? st[(NS + a * DIM + d) * NN + i] + st[(NS + a * DIM + d) * NN + j]
-                                      : Ge[a * DIM + d];
-            v = fma(gad, rr[a], v);
+            for (int a = 0; a < DIM; ++a) un = a ? fma(D[a], U[r][a] + UB[a], un) : D[a] * (U[r][a] + UB[a]);
+            const double F0 = rl[r] * un;
+            a0[r] += F0;
+            aE[r] = fma(fma(rl[r], ib[r] * pf[r], pa[r]), un, aE[r]);
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) {
+              am[r][d] = fma(F0, B.h[d], am[r][d]);
+              ap[r][d] = fma(pa[r], D[d], ap[r][d]);  // contravariant
+            }
+          } else {
+            double nv[DIM], ub[DIM], un = 0.0, hv = 0.0;
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) {
+              nv[d] = 0.0;
+#pragma unroll
+              for (int a = 0; a < DIM; ++a) {
+                const double gad = CURVED ? st[C::oG + (a * DIM + d) * Nq + ir[r]] +
+                                                st[C::oG + (a * DIM + d) * Nq + j]
+                                          : Ge[a * DIM + d];
+                nv[d] = a ? fma(gad, D[a], nv[d]) : gad * D[a];
+              }
+              ub[d] = ah[r][d] + B.h[d];
+              un = d ? fma(ub[d], nv[d], un) : ub[d] * nv[d];
+              hv = d ? fma(2.0 * ah[r][d], B.h[d], hv) : 2.0 * ah[r][d] * B.h[d];
+            }
+            const double F0 = rl[r] * un;
+            a0[r] += F0;
+            aE[r] = fma(fma(rl[r], fma(ib[r], pf[r], hv), pa[r]), un, aE[r]);
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) am[r][d] = fma(F0, ub[d], fma(pa[r], nv[d], am[r][d]));
           }
-          nv[r][d] = v;
         }
       }
-      ecflux_n_warp_hR<DIM, R, SMALL>(A, B, nv, P, F);
+      if (SPLIT) {  // sum pa n = G^T (contravariant sum)
 #pragma unroll
-      for (int r = 0; r < R; ++r)
+        for (int r = 0; r < R; ++r) {
+          double v[DIM];
 #pragma unroll
-        for (int q = 0; q < Nf; ++q) acc[r][q] += F[r][q];
+          for (int d = 0; d < DIM; ++d) {
+            v[d] = 0.0;
+#pragma unroll
+            for (int a = 0; a < DIM; ++a)
+              v[d] = fma(sNrm[e * SN + El::Nfaces * DIM + a * DIM + d], ap[r][a], v[d]);
+          }
+#pragma unroll
+          for (int d = 0; d < DIM; ++d) ap[r][d] = v[d];
+        }
+      }
     }
 
     // volume-face pairs, each evaluated once: warp h takes its face nodes
-    const int nfh = T::nf(h), f0h = T::f0(h);
-    const double *w1h = sW1 + R * L * f0h, *w2h = sW2 + R * L * f0h;
-    for (int s = 0; s < nfh; ++s) {
-      int ff = l + s;
-      if (ff >= nfh) ff -= nfh;
-      const int f = f0h + ff;
-      const NodeState<DIM> B = load(st, Nq + f);
-      const int fc = f / Nfq;
-      double nv[DIM];
-      if (!CURVED) {
+#pragma unroll 1
+    for (int fb = T::f0(h); fb < T::f0(h) + T::nf(h); fb += FACES ? Nfq : NF) {
+      const int n = FACES ? Nfq : T::nf(h);
+      // per block (one face): the direction, or the row's part of it
+      double nb[DIM], xi[R], nr[R][DIM], pb[R];
+      if (SPLIT) {
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) nv[d] = sNrm[e * SN + fc * DIM + d];
+        for (int d = 0; d < DIM; ++d) nb[d] = sNrm[e * SN + fb / Nfq * DIM + d];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          pb[r] = xi[r] = 0.0;
+#pragma unroll
+          for (int d = 0; d < DIM; ++d) xi[r] = d ? fma(ah[r][d], nb[d], xi[r]) : ah[r][d] * nb[d];
+        }
+      } else if (CURVED && FACES) {
+        row_normals(st, ir, fb / Nfq, nr);
       }
-      double af[Nf];
+      const double2 *wb = (const double2 *)sW + fb * R * L + l;
+#pragma unroll 1
+      for (int s = 0; s < n; ++s) {
+        int ff = l + s;
+        if (ff >= n) ff -= n;
+        const int f = fb + ff;
+        const Node B = load<TT>(st, Nq + f);
+        pair_means<R, TT>(ahr, ab, alr, alb, B.hr, B.b, B.lr, B.lb, P, rl, pa, ib, pf);
+        if (SPLIT) {
+          const double x = DIM == 3 ? B.x : st[C::oX + f];
+          double g0, gp, gE, gm[DIM];
 #pragma unroll
-      for (int q = 0; q < Nf; ++q) af[q] = 0.0;
-      double nvr[R][DIM], F[R][Nf];
+          for (int r = 0; r < R; ++r) {
+            const double2 w = wb[(s * R + r) * L];
+            const double un = xi[r] + x, F0 = rl[r] * un;
+            const double f4u = fma(rl[r], ib[r] * pf[r], pa[r]) * un;
+            const double g1 = w.x * F0, g2 = w.y * F0;
+            a0[r] += g1;
+            pb[r] = fma(w.x, pa[r], pb[r]);
+            aE[r] = fma(w.x, f4u, aE[r]);
+            g0 = r ? g0 + g2 : g2;
+            gp = r ? fma(w.y, pa[r], gp) : w.y * pa[r];
+            gE = r ? fma(w.y, f4u, gE) : w.y * f4u;
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        if (CURVED) {
-          const int i = ir[r];
-#pragma unroll
-          for (int d = 0; d < DIM; ++d) {
-            double v = 0.0;
-#pragma unroll
-            for (int a = 0; a < DIM; ++a)
-              v = fma(st[(NS + a * DIM + d) * NN + i] + st[(NS + a * DIM + d) * NN + Nq + f],
-                      sNr[fc * DIM + a], v);
-            nvr[r][d] = v;
+            for (int d = 0; d < DIM; ++d) {
+              am[r][d] = fma(g1, B.h[d], am[r][d]);
+              gm[d] = r ? fma(g2, ah[r][d], gm[d]) : g2 * ah[r][d];
+            }
           }
+          double2 *q = (double2 *)acc_f + f;
+          const double2 q0 = q[0], q1 = q[NF];
+          if (DIM == 3) {
+            const double2 q2 = q[2 * NF];
+            q[2 * NF] = make_double2(q2.x + gm[DIM - 1], q2.y + gE);
+          } else {
+            acc_f[4 * NF + f] += gE;
+          }
+          q[0] = make_double2(q0.x + g0, q0.y + gp);
+          q[NF] = make_double2(q1.x + gm[0], q1.y + gm[1]);
         } else {
+          double af[Nf], nfv[DIM];
+          if (!FACES && CURVED) row_normals(st, ir, f / Nfq, nr);
 #pragma unroll
-          for (int d = 0; d < DIM; ++d) nvr[r][d] = nv[d];
+          for (int d = 0; d < DIM; ++d)
+            nfv[d] = CURVED ? st[C::oN + d * NF + f] : sNrm[e * SN + f / Nfq * DIM + d];
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const double2 w = wb[(s * R + r) * L];
+            double nv[DIM], ub[DIM], un = 0.0, hv = 0.0, Fr[Nf];
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) {
+              nv[d] = CURVED ? nr[r][d] + nfv[d] : nfv[d];
+              ub[d] = ah[r][d] + B.h[d];
+              un = d ? fma(ub[d], nv[d], un) : ub[d] * nv[d];
+              hv = d ? fma(2.0 * ah[r][d], B.h[d], hv) : 2.0 * ah[r][d] * B.h[d];
+            }
+            Fr[0] = rl[r] * un;
+            Fr[DIM + 1] = fma(rl[r], fma(ib[r], pf[r], hv), pa[r]) * un;
+            a0[r] = fma(w.x, Fr[0], a0[r]);
+            aE[r] = fma(w.x, Fr[DIM + 1], aE[r]);
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) {
+              Fr[1 + d] = fma(Fr[0], ub[d], pa[r] * nv[d]);
+              am[r][d] = fma(w.x, Fr[1 + d], am[r][d]);
+            }
+#pragma unroll
+            for (int q = 0; q < Nf; ++q) af[q] = r ? fma(w.y, Fr[q], af[q]) : w.y * Fr[q];
+          }
+#pragma unroll
+          for (int q = 0; q < Nf; ++q) acc_f[q * NF + f] += af[q];
+        }
+        __syncwarp();
+      }
+      if (SPLIT) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+          for (int d = 0; d < DIM; ++d) ap[r][d] = fma(pb[r], nb[d], ap[r][d]);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      F[r][0] = a0[r];
+      F[r][DIM + 1] = aE[r];
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) {
+        F[r][1 + d] = am[r][d];
+        if (SPLIT) {
+          F[r][1 + d] = fma(ah[r][d], a0[r], am[r][d] + ap[r][d]);
+          F[r][DIM + 1] = fma(2.0 * ah[r][d], am[r][d], F[r][DIM + 1]);
         }
       }
-      ecflux_n_warp_hR<DIM, R, SMALL>(A, B, nvr, P, F);
+    }
+  }
+
+  // curved: n_i = sum_a nr_a G^a_i / 2 of the lane's rows for one face
+  __device__ __forceinline__ void row_normals(const double *st, const int (&ir)[R], int fc,
+                                              double (&nr)[R][DIM]) const {
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const double w1 = w1h[(r * nfh + s) * L + l];
-        const double w2 = w2h[(r * nfh + s) * L + l];
+    for (int r = 0; r < R; ++r)
 #pragma unroll
-        for (int q = 0; q < Nf; ++q) {
-          acc[r][q] = fma(w1, F[r][q], acc[r][q]);
-          af[q] = fma(w2, F[r][q], af[q]);
-        }
+      for (int d = 0; d < DIM; ++d) {
+        nr[r][d] = 0.0;
+#pragma unroll
+        for (int a = 0; a < DIM; ++a)
+          nr[r][d] = fma(st[C::oG + (a * DIM + d) * Nq + ir[r]], sNr[fc * DIM + a], nr[r][d]);
       }
+  }
+
+  // the face row f of element ee that the pair phase has summed
+  __device__ __forceinline__ void face_row(int ee, int f, double (&v)[Nf]) const {
+    const double *acc_f = sAcc + ee * SA;
+    if (!SPLIT) {
 #pragma unroll
-      for (int q = 0; q < Nf; ++q) acc_f[q * NF + f] += af[q];
-      __syncwarp();
+      for (int q = 0; q < Nf; ++q) v[q] = acc_f[q * NF + f];
+      return;
+    }
+    const double *st = sSt + ee * SE, *nb = sNrm + ee * SN + f / Nfq * DIM;
+    const double2 *q = (const double2 *)acc_f + f;
+    const double2 q0 = q[0], q1 = q[NF], hb = ((const double2 *)(st + C::oB))[Nq + f];
+    double m[DIM], hf[DIM], gE;
+    m[0] = q1.x;
+    m[1] = q1.y;
+    hf[0] = hb.x;
+    hf[1] = hb.y;
+    if (DIM == 3) {
+      const double2 q2 = q[2 * NF];
+      m[DIM - 1] = q2.x;
+      gE = q2.y;
+      hf[DIM - 1] = st[C::oC + 2 * (Nq + f)];
+    } else {
+      gE = acc_f[4 * NF + f];
+    }
+    v[0] = q0.x;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      v[1 + d] = fma(hf[d], q0.x, fma(nb[d], q0.y, m[d]));
+      gE = fma(2.0 * hf[d], m[d], gE);
+    }
+    v[DIM + 1] = gE;
+  }
+
+  // a face row back into its slots, for the lift
+  __device__ __forceinline__ void put_row(int ee, int f, const double (&v)[Nf]) const {
+    double *acc_f = sAcc + ee * SA;
+    if (SPLIT) {
+      double2 *q = (double2 *)acc_f + f;
+      q[0].x = v[0];
+      q[NF] = make_double2(v[1], v[2]);
+      if (DIM == 3)
+        q[2 * NF] = make_double2(v[3], v[Nf - 1]);
+      else
+        acc_f[4 * NF + f] = v[Nf - 1];
+    } else {
+#pragma unroll
+      for (int q = 0; q < Nf; ++q) acc_f[q * NF + f] = v[q];
+    }
+  }
+  __device__ __forceinline__ void get_row(const double *acc_f, int f, double (&v)[Nf]) const {
+    if (SPLIT) {
+      const double2 *q = (const double2 *)acc_f + f;
+      v[0] = q[0].x;
+      const double2 q1 = q[NF];
+      v[1] = q1.x;
+      v[2] = q1.y;
+      if (DIM == 3) {
+        const double2 q2 = q[2 * NF];
+        v[3] = q2.x;
+        v[Nf - 1] = q2.y;
+      } else {
+        v[Nf - 1] = acc_f[4 * NF + f];
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < Nf; ++q) v[q] = acc_f[q * NF + f];
     }
   }
 
   // surface flux + Lax-Friedrichs penalty at the face points of the group's
   // batch elements [e0, e0 + G) (the TS threads t0, t0 + TS, ... of the
-  // group), added to the face-row accumulators: sf = rhsQf + 1/2
+  // group), added to the face rows: sf = rhsQf + 1/2
   // F_S(u-, u+).nJ - tau/4 max(lam-, lam+) sJ (u+ - u-) (Euler3D.okl:3256-3346,
-  // Euler2D.okl:1373-1453).  The minus state is the pair phase's node state
-  // (velocity stored halved) and the trace in uf; the plus trace is gathered
+  // Euler2D.okl:1373-1453).  The plus trace is gathered
   // from uf through mapPq (the neighbour indices of all of a thread's face
   // points are loaded first).
   template <int TS>
@@ -389,21 +709,19 @@ struct VolPairs {
         UM[q] = uf[idM + q * NF];
         UP[q] = uf[idP[u] + q * NF];
       }
-      NodeState<DIM> M = load(sSt + ee * SE, Nq + f);
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) M.vel[d] *= 2.0;  // the pair phase's states hold u/2
       double kM, kP, c2M, c2P;
-      node_state_surf<DIM>(UM, 1, P, kM, c2M);
+      const NodeState<DIM> M = node_state_surf<DIM>(UM, 1, P, kM, c2M);
       const NodeState<DIM> Pp = node_state_surf<DIM>(UP, 1, P, kP, c2P);
-      double F[Nf];
+      double F[Nf], v[Nf];
       ecflux_n_nolog<DIM>(M, Pp, nJ, P, F);
       const double lamM = fsqrt(kM) + fsqrt(c2M);
       const double lamP = fsqrt(kP) + fsqrt(c2P);
       const double tau = (DIM == 3) ? P.tau : 1.0;
       const double Lfc = tau * 0.25 * fmax(lamM, lamP) * sJ;
-      double *a0 = sAcc + ee * SA;
+      face_row(ee, f, v);
 #pragma unroll
-      for (int q = 0; q < Nf; ++q) a0[q * NF + f] = a0[q * NF + f] + 0.5 * F[q] - Lfc * (UP[q] - UM[q]);
+      for (int q = 0; q < Nf; ++q) v[q] = v[q] + 0.5 * F[q] - Lfc * (UP[q] - UM[q]);
+      put_row(ee, f, v);
     }
   }
 
@@ -411,54 +729,66 @@ struct VolPairs {
   // the group splitting the face nodes as in the pair phase
   __device__ __forceinline__ void lift(double (&acc)[R][Nf]) const {
     const double *sf = sAcc + e * SA;
-    const int nfh = T::nf(h), f0h = T::f0(h);
-    const double *w1h = sW1 + R * L * f0h;
-    for (int s = 0; s < nfh; ++s) {
-      int ff = l + s;
-      if (ff >= nfh) ff -= nfh;
-      const int f = f0h + ff;
+#pragma unroll 1
+    for (int fb = T::f0(h); fb < T::f0(h) + T::nf(h); fb += FACES ? Nfq : NF) {
+      const int n = FACES ? Nfq : T::nf(h);
+      const double *wb = sW + 2 * (fb * R * L + l);
+      for (int s = 0; s < n; ++s) {
+        int ff = l + s;
+        if (ff >= n) ff -= n;
+        double v[Nf];
+        get_row(sf, fb + ff, v);
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const double w = 2.0 * w1h[(r * nfh + s) * L + l];
+        for (int r = 0; r < R; ++r) {
+          const double w = 2.0 * wb[2 * (s * R + r) * L];
 #pragma unroll
-        for (int q = 0; q < Nf; ++q) acc[r][q] = fma(w, sf[q * NF + f], acc[r][q]);
+          for (int q = 0; q < Nf; ++q) acc[r][q] = fma(w, v[q], acc[r][q]);
+        }
       }
     }
   }
 
-  // warp 1 parks its partial rows in element e's state block ([Nf][Nq]);
-  // call between two __syncthreads
   // the per-node logarithms of the batch elements [e0, e0 + ne) (threads t0,
-  // t0 + ts, ...), from the stored density and beta: the same values the
-  // prologue's node_state would have stored
+  // t0 + ts, ...), from the stored density and beta
   __device__ __forceinline__ void fill_logs(int e0, int ne, int t0, int ts) const {
     for (int t = t0; t < ne * NN; t += ts) {
       double *st = sSt + (e0 + t / NN) * SE;
       const int n = t % NN;
-      st[(DIM + 2) * NN + n] = log(st[n]);
-      st[(DIM + 3) * NN + n] = log(st[(DIM + 1) * NN + n]);
+      const double2 a = ((const double2 *)(st + C::oA))[n];
+      ((double2 *)st)[n] = make_double2(log(2.0 * a.x), log(a.y));
     }
   }
 
   // The pair phase of the group (H warps, threads t0 .. t0 + ts - 1 over
-  // the batch elements [e0, e0 + G), `gsync` its barrier), after a prologue
-  // without logarithms: where every pair of the group's elements is nearly
-  // equal (small_pairs) the pairs take the u^2 series with no vote and need
-  // no logarithm; otherwise the logarithms are filled in first (they feed
-  // the log-difference branch).
+  // the batch elements [e0, e0 + G), `gsync` its barrier): the pair loops of
+  // the range that the group's states span; the logarithms only where the
+  // log-difference may be needed.
   template <typename Sync>
   __device__ __forceinline__ void group_pairs(double (&acc)[R][Nf], const Phys &P, int e0, int t0,
                                               int ts, Sync gsync) const {
-    if (small_pairs<DIM, NN, L>(sSt + e * SE, l)) {
-      pairs<true>(acc, P);
+    const double *st = sSt + e * SE;
+    const int range = state_range<NN, L>(l, [&](int n, double &r, double &b) {
+      const double2 a = ((const double2 *)(st + C::oA))[n];
+      r = a.x;
+      b = a.y;
+    });
+    if (range == 0) {
+      pairs<0>(acc, P);
+    } else if (range == 1) {
+      pairs<1>(acc, P);
+    } else if (range == 2) {
+      pairs<2>(acc, P);
     } else {
       fill_logs(e0, G, t0, ts);
       gsync();
-      pairs<false>(acc, P);
+      pairs<3>(acc, P);
     }
   }
 
+  // warp 1 parks its partial rows in element e's state block (over the
+  // logarithms and densities, [Nf][Nq]; the group's pairs are done)
   __device__ __forceinline__ void park_rows(const double (&acc)[R][Nf]) const {
+    static_assert(Nf * Nq <= 4 * NN, "row buffer");
     double *rowbuf = sSt + e * SE;
     if (h == 1) {
 #pragma unroll
@@ -511,12 +841,18 @@ vol_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
   };
   // stage the group's elements from kq on (face traces, a contiguous range
   // of Qf) into shared memory
+  // (without room for them: into L2), and the affine elements' geometric factors
   auto prefetch_group = [&](int kq) {
     if (kq < K) {
       const int n = min(K - kq, G) * NF * Nf;
       const double *src = Qf + (size_t)kq * NF * Nf;
-      double *dst = v.sPre + (size_t)q * G * NF * Nf;
-      for (int t = tq; t < n; t += GT) cp_async8(dst + t, src + t);
+      if (PRE) {
+        double *dst = v.sPre + (size_t)q * G * NF * Nf;
+        for (int t = tq; t < n; t += GT) cp_async8(dst + t, src + t);
+      } else {
+        for (int t = tq * 16; t < n; t += GT * 16) prefetch_l2(src + t);
+      }
+      v.fetch_geo(K, kq - q * G, q * G, tq, GT, vgeo);
     }
     cp_async_commit();
   };
@@ -538,11 +874,11 @@ vol_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
     return (blist ? blist[cb] : cb) * E + (g - cb * NG) * G;
   };
   const int g0 = q * (int)gridDim.x + (int)blockIdx.x;
-  if (PRE) prefetch_group(slice(g0));
+  prefetch_group(slice(g0));
 
   for (int gi = g0; gi < ns; gi += sstep) {
     const int kg = slice(gi);
-    if (PRE) cp_async_wait_all();
+    cp_async_wait_all();
     // a slice whose elements all lie past the end (of a partial last batch)
     // has nothing to compute, and must not read element K-1's input, which
     // the group owning it may already have overwritten with its RHS
@@ -550,17 +886,26 @@ vol_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
     // the helpers index the group's elements as k0 + q G + (0 .. G-1)
     const int k0 = kg - q * G;
     gsync();  // the group's traces staged / its previous slice done with its shared memory
-    v.template prologue_group<false, GT>(K, k0, q * G, tq, vgeo, vfgeo, rhsQ, Qf, P,
-                                         PRE ? v.sPre : nullptr);
+    v.template prologue_group<GT>(K, k0, q * G, tq, vgeo, vfgeo, rhsQ, Qf, P, PRE ? v.sPre : nullptr);
     gsync();
-    if (PRE) prefetch_group(slice(gi + sstep));  // the next slice's traces, during the pairs
+    prefetch_group(slice(gi + sstep));  // the next slice's traces, during the pairs
     double acc[R][Nf];
     v.group_pairs(acc, P, q * G, tq, GT, gsync);
-    gsync();  // the group's pairs done: its state block becomes the row buffer
+    gsync();  // the group's pairs done
     if (SURF) {
       v.template surface<GT>(K, k0, q * G, tq, fgeo, mapPq, Qf, P);
-      gsync();  // face rows complete (and the states read): lift, then park
+      gsync();  // face rows complete: lift
       v.lift(acc);
+    } else {
+      for (int t = tq; t < G * NF; t += GT) {
+        const int ee = q * G + t / NF, f = t % NF;
+        if (k0 + ee >= K) continue;
+        double row[Nf];
+        v.face_row(ee, f, row);
+        double *outf = rhsQf + (size_t)(k0 + ee) * NF * Nf + f;
+#pragma unroll
+        for (int c = 0; c < Nf; ++c) outf[c * NF] = row[c];
+      }
     }
     v.park_rows(acc);
     gsync();
@@ -577,11 +922,6 @@ vol_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
             for (int q = 0; q < Nf; ++q) out[q * Nq] = H == 2 ? acc[r][q] + rowbuf[q * Nq + i] : acc[r][q];
           }
         }
-      }
-      if (!SURF) {
-        const double *a0 = v.sAcc + v.e * V::SA;
-        double *outf = rhsQf + (size_t)k * NF * Nf;
-        for (int t = v.h * L + v.l; t < NF * Nf; t += H * L) outf[t] = a0[t];
       }
     }
   }

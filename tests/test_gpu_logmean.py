@@ -154,3 +154,40 @@ def test_volume_kernel_per_warp_log_mean_paths(cuda, dim, N, curved, targets):
     d.sync()
     h = d.get(s)
     assert rel(h["rhsQ"], ref["rhsQ"]) < RTOL, rel(h["rhsQ"], ref["rhsQ"])
+
+
+@pytest.mark.parametrize("dim,N,curved", [(3, 1, False), (3, 2, False), (3, 3, False), (3, 4, False),
+                                          (3, 2, True), (3, 4, True), (2, 1, False), (2, 2, False),
+                                          (2, 3, False), (2, 4, False), (2, 3, True), (2, 4, True)])
+@pytest.mark.parametrize("edge", [1.3e-5, 2e-3, 6e-2])
+def test_volume_kernel_either_side_of_a_polynomial_range(cuda, dim, N, curved, edge):
+    """The log-mean's polynomials hold up to u = 1.3e-5, 2e-3 and 6e-2 (beyond
+    it, the difference of logarithms), chosen per warp by its elements'
+    largest u: element lists whose warps lie below, above and on both sides of
+    each edge.  Both kernels must equal the reference's to 1e-12."""
+    mesh = M.periodic_cube(3, warp=M.warp_cube(0.05) if curved else None) if dim == 3 \
+        else M.periodic_square(12, 13)
+    geo = M.build_geometry(mesh, N)
+    # long runs of equal targets: whole warps (of up to 32 elements) on one side
+    targets = np.repeat([0.3 * edge, 0.45 * edge, 4.0 * edge, 0.5 * edge], 48)
+    targets[96 + 48 + 20] = 5.0 * edge
+    uq, uf, rho, beta = warp_regime_state(geo, 11 * dim + N, targets)
+    ue = np.maximum(element_u(rho), element_u(beta))
+    assert (ue[:geo.K] < edge).any() and (ue > edge).any()
+    d = Dev(cuda, geo, curved)
+    st = dict(rhsQ=uq, Qf=uf, rhsQf=np.zeros_like(uf))
+    ref = {k: v.copy() for k, v in st.items()}
+    O_ = oracle(geo.ops, curved)
+    O_.vol(geo, ref["Qf"], ref["rhsQ"], ref["rhsQf"])
+    s = d.put(st)
+    d.vol(s)
+    d.sync()
+    h = d.get(s)
+    assert rel(h["rhsQ"], ref["rhsQ"]) < RTOL, rel(h["rhsQ"], ref["rhsQ"])
+    assert rel(h["rhsQf"], ref["rhsQf"]) < RTOL, rel(h["rhsQf"], ref["rhsQf"])
+    O_.surf(geo, np.ascontiguousarray(st["Qf"]).copy(), ref["rhsQf"], ref["rhsQ"])
+    s = d.put(st)
+    d.volsurf(s)
+    d.sync()
+    h = d.get(s)
+    assert rel(h["rhsQ"], ref["rhsQ"]) < RTOL, rel(h["rhsQ"], ref["rhsQ"])
