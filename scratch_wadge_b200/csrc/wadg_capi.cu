@@ -79,6 +79,17 @@ int persistent_grid(int K, int E, size_t smem) {
   return batches < num_sms() * per_sm ? batches : num_sms() * per_sm;
 }
 
+// CTAs of the volume kernel: its element groups take slices of G elements, slice
+// s going to CTA s mod grid first, so one CTA per slice up to the resident
+// number: a mesh of few slices runs one group on each of many SMs rather than
+// all of a CTA's groups on few (10 time steps, one CTA per batch before: 162 tets
+// N=2 1.39 -> 1.03 ms, 2146 curved triangles N=4 1.57 -> 1.42 ms, 2048 triangles
+// N=3 1.01 -> 0.94 ms)
+template <class C>
+int vol_grid(int K) {
+  return persistent_grid(K, C::T::G, C::smem_vol);
+}
+
 // candidate CTA shapes of the pair volume kernel (warps per CTA; elements per
 // CTA = warps / 2 * 32 / lanes per element): the default, then two and four
 // warps fewer.  In 2D the second is 16 warps where they fit: four fields need
@@ -151,7 +162,7 @@ int launch_vol_pairs_w(const wadg_ctx *c, int K, const double *vgeo, const doubl
     if (e != cudaSuccess) return cuda_check(e, "volume kernel smem attribute");
     attr.here() = true;
   }
-  const int grid = persistent_grid(K, C::E, C::smem_vol);
+  const int grid = vol_grid<C>(K);
   kern<<<grid, C::threads, C::smem_vol, c->stream>>>(K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq,
                                                       VqLq, VfPq, Qf, rhsQ, rhsQf, c->phys, fgeo,
                                                       mapPq, blist, nb);
@@ -301,7 +312,7 @@ template <int DIM, int N, bool CURVED, int W, int RR = 0>
 void vol_shape(int K, int *E, int *grid) {
   using C = VolPairsCfg<DIM, N, CURVED, W, RR>;
   *E = C::E;
-  *grid = persistent_grid(K, C::E, C::smem_vol);
+  *grid = vol_grid<C>(K);
 }
 
 template <int DIM, int N, bool CURVED>
