@@ -33,7 +33,7 @@ def build(force=False, verbose=False, extra=()):
     procs = []
     for src in sources():
         obj = os.path.join(bdir, os.path.basename(src) + ".o")
-        cmd = [NVCC, "-O3", "-std=c++17", *ARCH, "-lineinfo", "-Xcompiler", "-fPIC", "--split-compile=0",
+        cmd = [NVCC, "-O3", "-std=c++17", *ARCH, "-lineinfo", "-Xcompiler", "-fPIC",
                "-Xptxas", "-v" if verbose else "-O3", "-I", os.path.join(ROOT, "include"),
                "-c", src, "-o", obj, *extra]
         procs.append((cmd, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))

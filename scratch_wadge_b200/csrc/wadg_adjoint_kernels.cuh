@@ -627,9 +627,9 @@ adj_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
       }
     }
     };
-    const double spread = state_spread<NN, L>(l, [&](int n, double &r, double &b) {
-      r = st[n];
-      b = st[(DIM + 1) * NN + n];
+    const double spread = state_spread<NN, L>(l, [&](int n, int &r, int &b) {
+      r = __double2hiint(st[n]);
+      b = __double2hiint(st[(DIM + 1) * NN + n]);
     });
     if (__all_sync(0xffffffffu, spread < SMALL_U))
       pair_loops(BoolTag<true>());

@@ -47,6 +47,10 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 __device__ __forceinline__ void prefetch_l2(const void *p) {
   asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p));
 }
+// the lines of `bytes` bytes from p on, by threads t0, t0 + ts, ...
+__device__ __forceinline__ void prefetch_lines(const void *p, int bytes, int t0, int ts) {
+  for (int t = t0 * 128; t < bytes; t += ts * 128) prefetch_l2((const char *)p + t);
+}
 
 struct Phys {
   double gamma;
@@ -230,33 +234,40 @@ __device__ __forceinline__ void UV(const double *V, double *U, const Phys &P) {
 // The largest u = ((a-b)/(a+b))^2, for the density and for beta, over every
 // pair that a lane's element forms, volume-volume and volume-face: over the
 // element's nodes it belongs to the extreme pair, ((max - min)/(max + min))^2.
-// The L lanes of an element reduce by shuffles; node(n, rho, beta) gives node
-// n's density and beta up to constant factors.  Infinite where a state is not
-// positive.  Must be called by all 32 lanes of the warp.
+// The extremes are taken of the high words (as integers: positive doubles sort
+// as their bits do), with the low words that make u larger: high by up to 2e-6
+// of max + min.  The L lanes of an element reduce by shuffles; node(n, rho,
+// beta) gives the high words of node n's density and beta up to constant
+// factors.  Infinite where a state is not positive or not finite.  Must be
+// called by all 32 lanes of the warp.
 template <int NN, int L, typename Node>
 __device__ __forceinline__ double state_spread(int l, Node node) {
-  double rmin, rmax, bmin, bmax;
+  int rmin, rmax, bmin, bmax;
   node(l < NN ? l : 0, rmin, bmin);
   rmax = rmin;
   bmax = bmin;
+#pragma unroll 4
   for (int n = l + L; n < NN; n += L) {
-    double r, b;
+    int r, b;
     node(n, r, b);
-    rmin = fmin(rmin, r);
-    rmax = fmax(rmax, r);
-    bmin = fmin(bmin, b);
-    bmax = fmax(bmax, b);
+    rmin = min(rmin, r);
+    rmax = max(rmax, r);
+    bmin = min(bmin, b);
+    bmax = max(bmax, b);
   }
 #pragma unroll
   for (int o = L / 2; o >= 1; o >>= 1) {
-    rmin = fmin(rmin, __shfl_xor_sync(0xffffffffu, rmin, o));
-    rmax = fmax(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
-    bmin = fmin(bmin, __shfl_xor_sync(0xffffffffu, bmin, o));
-    bmax = fmax(bmax, __shfl_xor_sync(0xffffffffu, bmax, o));
+    rmin = min(rmin, __shfl_xor_sync(0xffffffffu, rmin, o));
+    rmax = max(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
+    bmin = min(bmin, __shfl_xor_sync(0xffffffffu, bmin, o));
+    bmax = max(bmax, __shfl_xor_sync(0xffffffffu, bmax, o));
   }
-  const double fr = (rmax - rmin) * rcp(rmax + rmin), fb = (bmax - bmin) * rcp(bmax + bmin);
-  // a NaN fails the comparisons
-  if (!(rmin > 0.0 && bmin > 0.0 && fr <= 1.0 && fb <= 1.0)) return INFINITY;
+  // sign bit: not positive (as an integer, below every positive high word);
+  // exponent all ones: infinite or NaN
+  if (rmin <= 0 || bmin <= 0 || rmax >= 0x7ff00000 || bmax >= 0x7ff00000) return INFINITY;
+  const double r0 = __hiloint2double(rmin, 0), r1 = __hiloint2double(rmax, -1);
+  const double b0 = __hiloint2double(bmin, 0), b1 = __hiloint2double(bmax, -1);
+  const double fr = (r1 - r0) * rcp(r1 + r0), fb = (b1 - b0) * rcp(b1 + b0);
   return fmax(fr * fr, fb * fb);
 }
 

@@ -1,0 +1,6 @@
+// the 2D kernels of degree 1
+#include "wadg_launch.cuh"
+
+namespace wadg {
+WADG_LAUNCHES_DEGREE(, 2, 1)
+}  // namespace wadg

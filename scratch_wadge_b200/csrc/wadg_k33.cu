@@ -1,0 +1,6 @@
+// the 3D kernels of degree 3
+#include "wadg_launch.cuh"
+
+namespace wadg {
+WADG_LAUNCHES_DEGREE(, 3, 3)
+}  // namespace wadg

@@ -1,0 +1,397 @@
+// Launches of the volume, surface, update and fused stage kernels: CTA shapes,
+// grids and the choice among them.  The function templates are instantiated
+// once per (dim, N) in wadg_k<dim><N>.cu, so that the degrees compile in
+// parallel; wadg_capi.cu calls them.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "../../include/wadg.h"
+#include "wadg_host.h"
+#include "wadg_stage.cuh"
+#include "wadg_surf_mma.cuh"
+#include "wadg_update_mma.cuh"
+#include "wadg_vol.cuh"
+
+struct wadg_ctx {
+  int dim, N, Nq, Nfq, Nfaces;
+  wadg::Phys phys;
+  cudaStream_t stream;
+  int vol_warps = 0;  // warps per CTA of the pair volume kernel; 0 = the default
+  int vol_rows = 0;   // rows per lane of its node-to-thread map; 0 = the default
+};
+
+namespace wadg {
+
+int fail(int code, const char *fmt, ...);  // wadg_capi.cu: sets wadg_last_error, returns code
+int cuda_check(cudaError_t e, const char *what);
+
+inline int after_launch(const char *name) { return cuda_check(cudaGetLastError(), name); }
+
+// warps per CTA of the pair-scheduled volume kernel: as many as fit in 227 KB
+// of shared memory, at most `cap`; from 8 on a multiple of 4, the same number on
+// each quarter of the SM (10 warps leave 3 on two of them and 168 registers per
+// thread as with 12, so they run as long as 12 would for 10/12 of the work: curved
+// 3D N=4, K=10368 0.40 ms with 10 warps, 0.33 with 8)
+template <int DIM, int N, bool CURVED, int RR = 0>
+constexpr int volpairsW_fit(int cap) {
+  using C = VolPairsCfg<DIM, N, CURVED, 2, RR>;
+  constexpr size_t per_warp = C::per_elem * VolTile<DIM, N, RR>::G / C::H;
+  constexpr size_t w = (227 * 1024 - C::fixed) / per_warp;
+  return w >= (size_t)cap ? cap : (w < 2 ? 2 : (int)(w < 8 ? w & ~size_t(1) : w & ~size_t(3)));
+}
+
+// the default shape: at most 12 warps (register budget ~170 per thread)
+template <int DIM, int N, bool CURVED>
+constexpr int volpairsW() {
+  return volpairsW_fit<DIM, N, CURVED>(12);
+}
+
+inline int num_sms() { return wadg_internal::sm_count(); }
+
+// a kernel on the context's stream
+template <class... KA, class... A>
+int launch(const wadg_ctx *c, void (*kern)(KA...), int grid, int threads, size_t smem, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  return cuda_check(cudaLaunchKernelEx(&cfg, kern, KA(args)...), "kernel launch");
+}
+
+// CTAs of a persistent kernel over K elements in batches of E: one per batch,
+// at most as many as are resident at once (shared memory per CTA `smem`); CTA
+// b takes batches b, b + grid, b + 2 grid, ...
+inline int persistent_grid(int K, int E, size_t smem) {
+  const int per_sm = (int)((227 * 1024) / smem) > 0 ? (int)((227 * 1024) / smem) : 1;
+  const int batches = (K + E - 1) / E;
+  return batches < num_sms() * per_sm ? batches : num_sms() * per_sm;
+}
+
+// CTAs of the volume kernel: its element groups take slices of G elements, slice
+// s going to CTA s mod grid first, so one CTA per slice up to one per SM, and
+// more per SM only when the slices outnumber those CTAs' groups: a mesh of few
+// slices runs one group on each of many SMs rather than all of a CTA's groups on
+// few (10 time steps, one CTA per batch before: 162 tets N=2 1.39 -> 1.03 ms,
+// 2146 curved triangles N=4 1.57 -> 1.42 ms, 2048 triangles N=3 1.01 -> 0.94 ms)
+template <class C>
+int vol_grid(int K) {
+  const int slices = (K + C::T::G - 1) / C::T::G, groups = C::threads / 32 / C::H;
+  if (slices <= num_sms() * groups) return slices < num_sms() ? slices : num_sms();
+  return persistent_grid(K, C::T::G, C::smem_vol);
+}
+
+// candidate CTA shapes of the pair volume kernel (warps per CTA; elements per
+// CTA = warps / 2 * 32 / lanes per element): the default, then two and four
+// warps fewer.  In 2D the second is 16 warps where they fit: four fields need
+// fewer registers (128 per thread), and large 2D meshes run fastest at 16,
+// small ones at 8
+template <int DIM, int N, bool CURVED>
+constexpr int volpairsW_cand(int i) {
+  constexpr int W0 = volpairsW<DIM, N, CURVED>();
+  constexpr int Wbig = DIM == 2 ? volpairsW_fit<DIM, N, CURVED>(16) : W0;
+  if (i == 1 && Wbig > W0) return Wbig;
+  return i == 0 ? W0 : (W0 - 2 * i >= 2 ? W0 - 2 * i : 0);
+}
+
+// The other node-to-thread maps: half and twice the default's lanes per
+// element (about twice and half its rows per lane), each given to the kernels
+// as RR = rows per lane.  A map is a candidate when it has as many lanes as
+// intended (2 to 32), keeps a face node per lane in each warp's face half,
+// pads no more node slots than the default, holds at most 4 rows per lane and
+// fits a CTA of at least 4 warps in shared memory.  (Six rows per lane need
+// more than 255 registers in 3D: 140-530 bytes of spills at every degree.)
+// alt_rows<DIM, N, CURVED, j>(), j = 0 (half the lanes) or 1 (twice): its RR,
+// or 0 when it is no candidate; its warps per CTA: the most that fit, up to 16
+// with at most two rows per lane, else 8 (up to 255 registers per thread).
+template <int DIM, int N, int RR>
+struct NodeMap {  // VolTile's arithmetic, without its static checks
+  static constexpr int Nq = Elem<DIM, N>::Nq;
+  static constexpr int Lraw = RR > 0 ? (Nq + RR - 1) / RR : (Nq + 2) / 3;
+  static constexpr int L = Lraw <= 1 ? 1 : Lraw <= 2 ? 2 : Lraw <= 4 ? 4 : Lraw <= 8 ? 8 : Lraw <= 16 ? 16 : 32;
+  static constexpr int R = (Nq + L - 1) / L;
+  static constexpr int pad = L * R - Nq;
+};
+template <int DIM, int N, bool CURVED, int RR>
+constexpr int alt_warps() {
+  return volpairsW_fit<DIM, N, CURVED, RR>(NodeMap<DIM, N, RR>::R <= 2 ? 16 : 8);
+}
+template <int DIM, int N, bool CURVED, int j>
+constexpr int alt_rows() {
+  constexpr int L0 = NodeMap<DIM, N, 0>::L, Lt = j == 0 ? L0 / 2 : 2 * L0;
+  if constexpr (Lt < 2 || Lt > 32) {
+    return 0;
+  } else {
+    constexpr int RR = (Elem<DIM, N>::Nq + Lt - 1) / Lt;
+    using M = NodeMap<DIM, N, RR>;
+    // (nf1: the smaller face half, the second warp's when there are two)
+    constexpr int nf1 = Elem<DIM, N>::NfqNf / 2;
+    constexpr int faces = nf1 >= M::L ? nf1 : Elem<DIM, N>::NfqNf;
+    if constexpr (M::L != Lt || faces < M::L || M::pad > NodeMap<DIM, N, 0>::pad || M::R > 4) {
+      return 0;
+    } else {
+      constexpr int W = alt_warps<DIM, N, CURVED, RR>();
+      return (W >= 4 && VolPairsCfg<DIM, N, CURVED, W, RR>::smem <= 227 * 1024) ? RR : 0;
+    }
+  }
+}
+
+// SURF: the volume + surface kernel (rhsQf unused; fgeo, mapPq read)
+template <int DIM, int N, bool CURVED, int W, bool SURF = false, int RR = 0, int HH = 0>
+int launch_vol_pairs_w(const wadg_ctx *c, int K, const double *vgeo, const double *vfgeo,
+                       const double *nrJ, const double *nsJ, const double *ntJ, const double *Drq,
+                       const double *Dsq, const double *Dtq, const double *VqLq, const double *VfPq,
+                       const double *Qf, double *rhsQ, double *rhsQf,
+                       const double *fgeo = nullptr, const uint32_t *mapPq = nullptr,
+                       const int *blist = nullptr, const int *nb = nullptr) {
+  using C = VolPairsCfg<DIM, N, CURVED, W, RR, HH>;
+  static_assert(C::smem_vol <= 227 * 1024, "pair-scheduled volume kernel does not fit in shared memory");
+  auto kern = vol_pairs_kernel<DIM, N, CURVED, W, SURF, RR, HH>;
+  static wadg_internal::PerDevice<bool> attr;
+  if (!attr.here()) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem_vol);
+    if (e != cudaSuccess) return cuda_check(e, "volume kernel smem attribute");
+    attr.here() = true;
+  }
+  const int grid = vol_grid<C>(K);
+  if (int r = launch(c, kern, grid, C::threads, C::smem_vol, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq,
+                     Dtq, VqLq, VfPq, Qf, rhsQ, rhsQf, c->phys, fgeo, mapPq, blist, nb))
+    return r;
+  return after_launch(SURF ? "volume + surface kernel" : "volume kernel");
+}
+
+// the volume + surface kernel in the context's CTA shape (wadg_ctx_set_vol_warps)
+template <int DIM, int N, bool CURVED>
+int launch_volsurf(const wadg_ctx *c, int K, const double *vgeo, const double *vfgeo,
+                   const double *fgeo, const uint32_t *mapPq, const double *nrJ,
+                   const double *nsJ, const double *ntJ, const double *Drq, const double *Dsq,
+                   const double *Dtq, const double *VqLq, const double *VfPq, const double *Qf,
+                   double *rhsQ, const int *blist = nullptr, const int *nb = nullptr) {
+  constexpr int A0 = alt_rows<DIM, N, CURVED, 0>(), A1 = alt_rows<DIM, N, CURVED, 1>();
+  if constexpr (A0 > 0)
+    if (c->vol_rows == A0)
+      return launch_vol_pairs_w<DIM, N, CURVED, alt_warps<DIM, N, CURVED, A0>(), true, A0>(
+          c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, nullptr, fgeo,
+          mapPq, blist, nb);
+  if constexpr (A1 > 0)
+    if (c->vol_rows == A1)
+      return launch_vol_pairs_w<DIM, N, CURVED, alt_warps<DIM, N, CURVED, A1>(), true, A1>(
+          c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, nullptr, fgeo,
+          mapPq, blist, nb);
+  constexpr int W1 = volpairsW_cand<DIM, N, CURVED>(1), W2 = volpairsW_cand<DIM, N, CURVED>(2);
+  if (W1 && c->vol_warps == W1)
+    return launch_vol_pairs_w<DIM, N, CURVED, (W1 ? W1 : 2), true>(
+        c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, nullptr, fgeo, mapPq,
+        blist, nb);
+  if (W2 && c->vol_warps == W2)
+    return launch_vol_pairs_w<DIM, N, CURVED, (W2 ? W2 : 2), true>(
+        c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, nullptr, fgeo, mapPq,
+        blist, nb);
+  return launch_vol_pairs_w<DIM, N, CURVED, volpairsW<DIM, N, CURVED>(), true>(
+      c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, nullptr, fgeo, mapPq,
+      blist, nb);
+}
+
+// the context's CTA shape (wadg_ctx_set_vol_warps), else the default
+template <int DIM, int N, bool CURVED>
+int launch_vol_pairs(const wadg_ctx *c, int K, const double *vgeo, const double *vfgeo,
+                     const double *nrJ, const double *nsJ, const double *ntJ, const double *Drq,
+                     const double *Dsq, const double *Dtq, const double *VqLq, const double *VfPq,
+                     const double *Qf, double *rhsQ, double *rhsQf) {
+  constexpr int A0 = alt_rows<DIM, N, CURVED, 0>(), A1 = alt_rows<DIM, N, CURVED, 1>();
+  if constexpr (A0 > 0)
+    if (c->vol_rows == A0)
+      return launch_vol_pairs_w<DIM, N, CURVED, alt_warps<DIM, N, CURVED, A0>(), false, A0>(
+          c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, rhsQf);
+  if constexpr (A1 > 0)
+    if (c->vol_rows == A1)
+      return launch_vol_pairs_w<DIM, N, CURVED, alt_warps<DIM, N, CURVED, A1>(), false, A1>(
+          c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, rhsQf);
+  constexpr int W1 = volpairsW_cand<DIM, N, CURVED>(1), W2 = volpairsW_cand<DIM, N, CURVED>(2);
+  if (W1 && c->vol_warps == W1)
+    return launch_vol_pairs_w<DIM, N, CURVED, (W1 ? W1 : 2)>(c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq,
+                                                             Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, rhsQf);
+  if (W2 && c->vol_warps == W2)
+    return launch_vol_pairs_w<DIM, N, CURVED, (W2 ? W2 : 2)>(c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq,
+                                                             Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, rhsQf);
+  return launch_vol_pairs_w<DIM, N, CURVED, volpairsW<DIM, N, CURVED>()>(
+      c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, rhsQf);
+}
+
+template <int DIM, int N, bool CURVED>
+int vol_warps_candidates(int *out) {
+  int n = 0;
+  for (int i = 0; i < 3; ++i)
+    if (int w = volpairsW_cand<DIM, N, CURVED>(i)) out[n++] = w;
+  return n;
+}
+
+// every compiled (warps, rows) shape: the default map's warps, then the
+// other maps (rows > 0)
+template <int DIM, int N, bool CURVED>
+int vol_shapes(int *warps, int *rows) {
+  int n = vol_warps_candidates<DIM, N, CURVED>(warps);
+  for (int i = 0; i < n; ++i) rows[i] = 0;
+  constexpr int A0 = alt_rows<DIM, N, CURVED, 0>(), A1 = alt_rows<DIM, N, CURVED, 1>();
+  if constexpr (A0 > 0) {
+    warps[n] = alt_warps<DIM, N, CURVED, A0>();
+    rows[n++] = A0;
+  }
+  if constexpr (A1 > 0) {
+    warps[n] = alt_warps<DIM, N, CURVED, A1>();
+    rows[n++] = A1;
+  }
+  return n;
+}
+
+template <int DIM, int N, bool CURVED>
+int launch_stage(const wadg_ctx *c, int K, const double *vgeo, const double *vfgeo,
+                 const double *fgeo, const uint32_t *mapPq, const double *nrJ, const double *nsJ,
+                 const double *ntJ, const double *Drq, const double *Dsq, const double *Dtq,
+                 const double *VqLq, const double *VfPq, const double *VqPq, const double *Jq,
+                 double fa, double fb, double fdt, const double *uq, const double *uf, double *Q,
+                 double *resQ, double *uq_out, double *uf_out) {
+  if (uf_out == uf) return fail(WADG_ERR_INVALID, "stage: uf_out must not be uf");
+  constexpr int W = stage_warps<DIM, N, CURVED, volpairsW<DIM, N, CURVED>()>();
+  using C = VolPairsCfg<DIM, N, CURVED, W>;
+  auto kern = stage_kernel<DIM, N, CURVED, W>;
+  static wadg_internal::PerDevice<bool> attr;
+  if (!attr.here()) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem_vol);
+    if (e != cudaSuccess) return cuda_check(e, "stage kernel smem attribute");
+    attr.here() = true;
+  }
+  const int grid = persistent_grid(K, C::E, C::smem_vol);
+  kern<<<grid, C::threads, C::smem_vol, c->stream>>>(K, vgeo, vfgeo, fgeo, mapPq, nrJ, nsJ, ntJ, Drq,
+                                                  Dsq, Dtq, VqLq, VfPq, VqPq, Jq, fa, fb, fdt, uq,
+                                                  uf, Q, resQ, uq_out, uf_out, c->phys);
+  return after_launch("stage kernel");
+}
+
+template <int DIM, int N>
+int launch_surf(const wadg_ctx *c, int K, const double *fgeo, const uint32_t *mapPq,
+                const double *VqLq, const double *Qf, const double *rhsQf, double *rhsQ) {
+  using C = SurfMmaCfg<DIM, N>;
+  if (int r = launch(c, surf_mma_kernel<DIM, N>, (K + C::EW - 1) / C::EW, C::threads, C::smem, K, fgeo,
+                     mapPq, VqLq, Qf, rhsQf, rhsQ, c->phys))
+    return r;
+  return after_launch("surf kernel");
+}
+
+// CTAs of the persistent update kernel: one per group of C::EW elements, at
+// most as many as are resident at once (occupancy, cached per device)
+template <int DIM, int N, bool CURVED>
+int update_grid(int K, int *grid) {
+  using C = UpdMmaCfg<DIM, N, CURVED>;
+  auto kern = update_mma_kernel<DIM, N, CURVED>;
+  static wadg_internal::PerDevice<int> per_sm_dev;
+  int &per_sm = per_sm_dev.here();
+  if (!per_sm) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem);
+    if (e != cudaSuccess) return cuda_check(e, "update kernel smem attribute");
+    int n = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, C::threads, C::smem);
+    if (e != cudaSuccess) return cuda_check(e, "update kernel occupancy");
+    per_sm = n < 1 ? 1 : n;
+  }
+  const int ctas = (K + C::EW - 1) / C::EW;
+  *grid = ctas < num_sms() * per_sm ? ctas : num_sms() * per_sm;
+  return WADG_OK;
+}
+
+// the launch shape of one kernel for K elements (wadg_kernel_shape)
+template <int DIM, int N, bool CURVED, int W, int RR = 0, int HH = 0>
+void vol_shape(int K, int *E, int *grid) {
+  using C = VolPairsCfg<DIM, N, CURVED, W, RR, HH>;
+  *E = C::E;
+  *grid = vol_grid<C>(K);
+}
+
+template <int DIM, int N, bool CURVED>
+int kernel_shape(const wadg_ctx *c, int kernel, int K, int *E, int *grid) {
+  constexpr int W1 = volpairsW_cand<DIM, N, CURVED>(1), W2 = volpairsW_cand<DIM, N, CURVED>(2);
+  constexpr int A0 = alt_rows<DIM, N, CURVED, 0>(), A1 = alt_rows<DIM, N, CURVED, 1>();
+  if ((kernel == WADG_KERNEL_VOL || kernel == WADG_KERNEL_VOLSURF) && c->vol_rows) {
+    if constexpr (A0 > 0)
+      if (c->vol_rows == A0) vol_shape<DIM, N, CURVED, alt_warps<DIM, N, CURVED, A0>(), A0>(K, E, grid);
+    if constexpr (A1 > 0)
+      if (c->vol_rows == A1) vol_shape<DIM, N, CURVED, alt_warps<DIM, N, CURVED, A1>(), A1>(K, E, grid);
+    return WADG_OK;
+  }
+  switch (kernel) {
+    case WADG_KERNEL_VOL:
+      if (W1 && c->vol_warps == W1) vol_shape<DIM, N, CURVED, (W1 ? W1 : 2)>(K, E, grid);
+      else if (W2 && c->vol_warps == W2) vol_shape<DIM, N, CURVED, (W2 ? W2 : 2)>(K, E, grid);
+      else vol_shape<DIM, N, CURVED, volpairsW<DIM, N, CURVED>()>(K, E, grid);
+      return WADG_OK;
+    case WADG_KERNEL_SURF:
+      *E = SurfMmaCfg<DIM, N>::EW;
+      *grid = (K + *E - 1) / *E;
+      return WADG_OK;
+    case WADG_KERNEL_UPDATE:
+      *E = UpdMmaCfg<DIM, N, CURVED>::EW;
+      return update_grid<DIM, N, CURVED>(K, grid);
+    case WADG_KERNEL_VOLSURF:  // the same CTA shapes as the volume kernel
+      if (W1 && c->vol_warps == W1) vol_shape<DIM, N, CURVED, (W1 ? W1 : 2)>(K, E, grid);
+      else if (W2 && c->vol_warps == W2) vol_shape<DIM, N, CURVED, (W2 ? W2 : 2)>(K, E, grid);
+      else vol_shape<DIM, N, CURVED, volpairsW<DIM, N, CURVED>()>(K, E, grid);
+      return WADG_OK;
+    case WADG_KERNEL_ADJ_PAIRS:
+      return wadg_internal::adj_pairs_shape(DIM, N, CURVED, K, E, grid);
+    case WADG_KERNEL_STAGE: {
+      using C = VolPairsCfg<DIM, N, CURVED, stage_warps<DIM, N, CURVED, volpairsW<DIM, N, CURVED>()>()>;
+      *E = C::E;
+      *grid = persistent_grid(K, C::E, C::smem_vol);
+      return WADG_OK;
+    }
+  }
+  return fail(WADG_ERR_INVALID, "unknown kernel %d", kernel);
+}
+
+template <int DIM, int N, bool CURVED>
+int launch_update(const wadg_ctx *c, int K, const double *Jq, const double *VqPq,
+                  const double *VfPq, double fa, double fb, double fdt, double *rhsQ,
+                  double *resQ, double *Q, double *Qf, const double *dtK = nullptr,
+                  const int *glist = nullptr, const int *ng = nullptr) {
+  using C = UpdMmaCfg<DIM, N, CURVED>;
+  static_assert(C::smem <= 227 * 1024, "update kernel does not fit in shared memory");
+  auto kern = update_mma_kernel<DIM, N, CURVED>;
+  int grid = 0;
+  if (int r = update_grid<DIM, N, CURVED>(K, &grid)) return r;
+  if (int r = launch(c, kern, grid, C::threads, C::smem, K, Jq, VqPq, VfPq, fa, fb, fdt, rhsQ, resQ, Q,
+                     Qf, c->phys, dtK, glist, ng))
+    return r;
+  return after_launch("update kernel");
+}
+
+// every launch of one (dim, N, curved), defined in wadg_k<dim><N>.cu
+#define WADG_LAUNCHES(X, D, N, C)                                                                  \
+  X template int launch_volsurf<D, N, C>(                                                          \
+      const wadg_ctx *, int, const double *, const double *, const double *, const uint32_t *,     \
+      const double *, const double *, const double *, const double *, const double *,              \
+      const double *, const double *, const double *, const double *, double *, const int *,       \
+      const int *);                                                                                \
+  X template int launch_vol_pairs<D, N, C>(                                                        \
+      const wadg_ctx *, int, const double *, const double *, const double *, const double *,       \
+      const double *, const double *, const double *, const double *, const double *,              \
+      const double *, const double *, double *, double *);                                         \
+  X template int launch_stage<D, N, C>(                                                            \
+      const wadg_ctx *, int, const double *, const double *, const double *, const uint32_t *,     \
+      const double *, const double *, const double *, const double *, const double *,              \
+      const double *, const double *, const double *, const double *, const double *, double,      \
+      double, double, const double *, const double *, double *, double *, double *, double *);     \
+  X template int launch_update<D, N, C>(const wadg_ctx *, int, const double *, const double *,     \
+                                        const double *, double, double, double, double *,          \
+                                        double *, double *, double *, const double *, const int *, \
+                                        const int *);                                              \
+  X template int kernel_shape<D, N, C>(const wadg_ctx *, int, int, int *, int *);                  \
+  X template int vol_warps_candidates<D, N, C>(int *);                                             \
+  X template int vol_shapes<D, N, C>(int *, int *);
+#define WADG_LAUNCHES_DEGREE(X, D, N)                                                              \
+  WADG_LAUNCHES(X, D, N, true)                                                                     \
+  WADG_LAUNCHES(X, D, N, false)                                                                    \
+  X template int launch_surf<D, N>(const wadg_ctx *, int, const double *, const uint32_t *,        \
+                                   const double *, const double *, const double *, double *);
+
+}  // namespace wadg

@@ -107,7 +107,7 @@ stage_kernel(int K, const double *__restrict__ vgeo, const double *__restrict__ 
         double *dst = v.sPre + (size_t)q * G * NF * Nf;
         for (int t = tq; t < n; t += GT) cp_async8(dst + t, src + t);
       } else {
-        for (int t = tq * 16; t < n; t += GT * 16) prefetch_l2(src + t);
+        prefetch_lines(src, n * 8, tq, GT);
       }
       v.fetch_geo(K, kb, q * G, tq, GT, vgeo);
     }
@@ -145,14 +145,13 @@ stage_kernel(int K, const double *__restrict__ vgeo, const double *__restrict__ 
       gsync();
       const int k = k0 + v.e;
       if (k < K && v.h == 0) {
-        const double *rowbuf = v.sSt + v.e * V::SE;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
           const int i = v.l + L * r;
           if (i < Nq) {
             double *out = uq_out + (size_t)k * Nq * Nf + i;
 #pragma unroll
-            for (int f = 0; f < Nf; ++f) out[f * Nq] = H == 2 ? acc[r][f] + rowbuf[f * Nq + i] : acc[r][f];
+            for (int f = 0; f < Nf; ++f) out[f * Nq] = v.row_sum(acc[r][f], f, i);
           }
         }
       }

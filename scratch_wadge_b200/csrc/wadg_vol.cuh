@@ -34,7 +34,7 @@
 // elements (one where a half of the face nodes would be fewer than L): each
 // walks its own volume columns and its own face nodes.  The face nodes come in
 // blocks: the warp's faces one after another where a face has at least L nodes
-// (FACES), else all of the warp's face nodes as one block.  At step s of a block
+// or the warps take one face each (FACES), else all of the warp's face nodes as one block.  At step s of a block
 // of n nodes lane l takes node (l + s) mod n, so the L lanes of a group always
 // touch L distinct face rows, and the two warps never the same one: both add
 // their R contributions to one copy of the face-row accumulators in shared
@@ -57,29 +57,37 @@ namespace wadg {
 // three rows per lane (L = the power of two >= Nq/3); RR > 0: about RR rows
 // (an autotuner candidate where it pads less, e.g. 2D N=4: Nq = 16 fills
 // L = 4 x 4 or 8 x 2 exactly, against 8 x 3 = 24 slots by default)
-template <int DIM, int N, int RR = 0> struct VolTile {
+// HH = 0: two warps per element group, or one; HH = Nfaces: a warp per face.
+template <int DIM, int N, int RR = 0, int HH = 0> struct VolTile {
   using El = Elem<DIM, N>;
   static constexpr int Lraw = RR > 0 ? (El::Nq + RR - 1) / RR : (El::Nq + 2) / 3;
   static constexpr int L = Lraw <= 1 ? 1 : Lraw <= 2 ? 2 : Lraw <= 4 ? 4 : Lraw <= 8 ? 8 : Lraw <= 16 ? 16 : 32;
   static constexpr int R = (El::Nq + L - 1) / L;
   static constexpr int G = 32 / L;  // elements per warp group
   static_assert(El::NfqNf >= L, "face schedule needs NfqNf >= L");
-  static constexpr int H = El::NfqNf / 2 >= L ? 2 : 1;  // warps per element group
-  static constexpr bool FACES = El::Nfq >= L;           // blocks of one face
-  // the face nodes of the two warps: whole faces where a block is one, else halves
-  static constexpr int nf0 = H == 1 ? El::NfqNf : FACES ? (El::Nfaces + 1) / 2 * El::Nfq : (El::NfqNf + 1) / 2;
-  __host__ __device__ static constexpr int nf(int h) { return h ? El::NfqNf - nf0 : nf0; }
-  __host__ __device__ static constexpr int f0(int h) { return h ? nf0 : 0; }
-  // the volume columns [c0(h), c0(h + 1)): so that both warps take about as many pairs
-  static constexpr int mid = (El::Nq + El::NfqNf) / 2 - nf0;
-  static constexpr int nc0 = H == 1 ? El::Nq : mid < 0 ? 0 : mid;
-  __host__ __device__ static constexpr int c0(int h) { return h == 0 ? 0 : h == 1 ? nc0 : El::Nq; }
+  static constexpr bool FACES = El::Nfq >= L || HH;  // blocks of one face
+  // steps of a block: a face of fewer nodes than lanes (2D N=4 with a warp per
+  // face) leaves the lanes past its end idle
+  static constexpr int NR = El::Nfq > L ? El::Nfq : L;
+  static constexpr int NP = FACES ? El::Nfaces * NR : El::NfqNf;  // (step, lane) pairs / L of all blocks
+  static constexpr int H = HH ? HH : El::NfqNf / 2 >= L ? 2 : 1;  // warps per element group
+  static_assert(HH == 0 || HH == El::Nfaces, "a warp per face, or the default");
+  // the face nodes [f0(h), f0(h + 1)) of warp h: whole faces where a block is one
+  __host__ __device__ static constexpr int f0(int h) {
+    return FACES ? (h * El::Nfaces + H - 1) / H * El::Nfq : (h * El::NfqNf + H - 1) / H;
+  }
+  __host__ __device__ static constexpr int nf(int h) { return f0(h + 1) - f0(h); }
+  // the volume columns [c0(h), c0(h + 1)): so that the warps take about as many steps each
+  __host__ __device__ static constexpr int c0(int h) {
+    const int c = h * (El::Nq + NP) / H - (FACES ? f0(h) / El::Nfq * NR : f0(h));
+    return c < 0 ? 0 : c > El::Nq ? El::Nq : c;
+  }
 };
 
-template <int DIM, int N, bool CURVED, int W, int RR = 0>
+template <int DIM, int N, bool CURVED, int W, int RR = 0, int HH = 0>
 struct VolPairsCfg {
   using El = Elem<DIM, N>;
-  using T = VolTile<DIM, N, RR>;
+  using T = VolTile<DIM, N, RR, HH>;
   static constexpr int H = T::H;                      // warps per element group
   static constexpr int threads = 32 * W;
   static constexpr int E = (W / H) * T::G;            // elements per batch
@@ -111,7 +119,7 @@ struct VolPairsCfg {
   // per-face nJ and G (affine), and the next slice's G
   static constexpr int SN = CURVED ? 0 : El::Nfaces * DIM + 2 * El::Nvgeo;
   static constexpr int nD = DIM * El::Nq * El::Nq;
-  static constexpr int nW = T::R * El::NfqNf * T::L;
+  static constexpr int nW = T::R * T::NP * T::L;
   static constexpr size_t fixed = sizeof(double) * (size_t)(nD + 2 * nW + El::Nfaces * DIM);
   static constexpr size_t per_elem = sizeof(double) * (size_t)(SE + SA + SN);
   static constexpr size_t smem = fixed + E * per_elem;
@@ -123,11 +131,11 @@ struct VolPairsCfg {
 };
 
 // Shared-memory carve-up and the phases common to the kernels.
-template <int DIM, int N, bool CURVED, int W, int RR = 0>
+template <int DIM, int N, bool CURVED, int W, int RR = 0, int HH = 0>
 struct VolPairs {
   using El = Elem<DIM, N>;
-  using T = VolTile<DIM, N, RR>;
-  using C = VolPairsCfg<DIM, N, CURVED, W, RR>;
+  using T = VolTile<DIM, N, RR, HH>;
+  using C = VolPairsCfg<DIM, N, CURVED, W, RR, HH>;
   static constexpr int Nq = El::Nq, NF = El::NfqNf, Nfq = El::Nfq, NN = El::NN;
   static constexpr int Nf = El::Nfields, NG = El::Nvgeo, L = T::L, R = T::R, G = T::G, E = C::E;
   static constexpr int SE = C::SE, SA = C::SA, SN = C::SN, H = C::H;
@@ -139,7 +147,7 @@ struct VolPairs {
 
   __device__ __forceinline__ VolPairs(double *smem) {
     sD = smem;                          // (Drq, Dsq) [2][j][i]
-    sW = sD + 2 * Nq * Nq;              // [2][node][R][L] 1/2 VqLq(i, f), -1/2 VfPq(f, i); 0 on padding rows
+    sW = sD + 2 * Nq * Nq;              // [2][block][step][R][L] 1/2 VqLq(i, f), -1/2 VfPq(f, i); 0 on padding rows
     sSt = sW + 2 * C::nW;               // [E][SE]     node states
     sAcc = sSt + E * SE;                // [E][SA]     face-row accumulators
     sD2 = sAcc + E * SA;                // Dtq [j][i]  (3D)
@@ -154,39 +162,39 @@ struct VolPairs {
     e = (warp / H) * G + g;
   }
 
-  // the block of face nodes that node p of the order [h][..] lies in: [fb, fb + n)
-  __device__ static __forceinline__ void block_of(int p, int &fb, int &n) {
-    if (FACES) {
-      fb = p / Nfq * Nfq;
-      n = Nfq;
-    } else {
-      const int hh = H == 2 && p >= T::nf0;
-      fb = T::f0(hh);
-      n = T::nf(hh);
-    }
+  // steps of the block at face node fb, and the node that lane l takes at step s
+  // (past a face's end: its last node, with weights 0 and no addition)
+  static constexpr bool IDLE = FACES && Nfq < L;
+  __device__ static __forceinline__ int steps(int h) { return FACES ? T::NR : T::nf(h); }
+  __device__ static __forceinline__ int node(int l, int s, int n) {
+    const int ff = l + s;
+    return ff >= n ? ff - n : ff;
+  }
+  __device__ static __forceinline__ int weights(int fb) {
+    return (FACES ? fb / Nfq * T::NR : fb) * R * L;
   }
 
   __device__ __forceinline__ void load_tables(const double *nrJ, const double *nsJ,
                                               const double *ntJ, const double *Drq,
                                               const double *Dsq, const double *Dtq,
                                               const double *VqLq, const double *VfPq) {
-    for (int t = tid; t < Nq * Nq; t += blockDim.x) {
+#pragma unroll 4
+    for (int t = tid; t < Nq * Nq; t += C::threads) {
       sD[2 * t] = Drq[t];
       sD[2 * t + 1] = Dsq[t];
       if (DIM == 3) sD2[t] = Dtq[t];
     }
-    for (int t = tid; t < C::nW; t += blockDim.x) {
+#pragma unroll 4
+    for (int t = tid; t < C::nW; t += C::threads) {
       const int ll = t % L, r = (t / L) % R, p = t / (L * R);
-      int fb, n;
-      block_of(p, fb, n);
-      const int i = ll + L * r;
-      int ff = ll + (p - fb);
-      if (ff >= n) ff -= n;
-      const int f = fb + ff;
-      sW[2 * t] = i < Nq ? 0.5 * VqLq[i + f * Nq] : 0.0;
-      sW[2 * t + 1] = i < Nq ? -0.5 * VfPq[f + i * NF] : 0.0;
+      const int hh = !FACES && H == 2 && p >= T::f0(1);
+      const int fb = FACES ? p / T::NR * Nfq : T::f0(hh);
+      const int i = ll + L * r, ff = node(ll, FACES ? p % T::NR : p - fb, steps(hh)), f = fb + ff;
+      const bool on = i < Nq && (!IDLE || ff < Nfq);
+      sW[2 * t] = on ? 0.5 * VqLq[i + f * Nq] : 0.0;
+      sW[2 * t + 1] = on ? -0.5 * VfPq[f + i * NF] : 0.0;
     }
-    for (int t = tid; t < El::Nfaces; t += blockDim.x) {
+    for (int t = tid; t < El::Nfaces; t += C::threads) {
       sNr[t * DIM + 0] = nrJ[t * Nfq];
       sNr[t * DIM + 1] = nsJ[t * Nfq];
       if (DIM == 3) sNr[t * DIM + 2] = ntJ[t * Nfq];
@@ -211,21 +219,17 @@ struct VolPairs {
   // element so that every lane computes on valid data.  ufs: the group's
   // face traces already staged in shared memory, or null.  The states carry
   // no logarithms (fill_logs adds them where a group needs
-  // them).  A thread's nodes go in chunks of four whose
-  // loads (global for the volume nodes) are all issued before their node
-  // states are computed.  The chunks run in a loop, not unrolled: unrolled,
-  // the 3D affine volume + surface kernel spilled registers (20 -> 64 bytes)
-  // and lost 2 %; rolled it gains 1.8 % there, 3 % in the affine volume
-  // kernel, and the same 2-7 % as unrolled in the curved and 2D kernels
+  // them).  The loads of a thread's nodes (global for the volume nodes) are
+  // issued before their node states are computed
   template <int TS>
   __device__ __forceinline__ void prologue_group(int K, int k0, int e0, int t0, const double *vgeo,
                                                  const double *vfgeo, const double *uq,
                                                  const double *uf, const Phys &P,
                                                  const double *ufs) {
     constexpr int NT = (G * NN + TS - 1) / TS;
-    // the thread's nodes in chunks of CH: a chunk's loads all in flight, few
-    // registers held
-    constexpr int CH = 4;  // 2, 3 and 4 measured: 4 is 0.3-2 % ahead
+    // the thread's nodes in chunks of CH, a chunk's loads all in flight: up to
+    // five nodes at once, more four at a time
+    constexpr int CH = NT <= 5 ? NT : 4;
 #pragma unroll 1
     for (int c0 = 0; c0 < NT; c0 += CH) {
       double u[CH][Nf];
@@ -407,7 +411,7 @@ struct VolPairs {
 #pragma unroll
         for (int c = 0; c < NG; ++c) Ge[c] = sNrm[e * SN + El::Nfaces * DIM + c];
       }
-      for (int j = T::c0(h); j < T::c0(h + 1 + (H == 1)); ++j) {
+      for (int j = T::c0(h); j < T::c0(h + 1); ++j) {
         const Node B = load<TT>(st, j);
         double UB[DIM];
         if (SPLIT) {
@@ -480,7 +484,7 @@ struct VolPairs {
     // volume-face pairs, each evaluated once: warp h takes its face nodes
 #pragma unroll 1
     for (int fb = T::f0(h); fb < T::f0(h) + T::nf(h); fb += FACES ? Nfq : NF) {
-      const int n = FACES ? Nfq : T::nf(h);
+      const int n = steps(h);
       // per block (one face): the direction, or the row's part of it
       double nb[DIM], xi[R], nr[R][DIM], pb[R];
       if (SPLIT) {
@@ -495,12 +499,11 @@ struct VolPairs {
       } else if (CURVED && FACES) {
         row_normals(st, ir, fb / Nfq, nr);
       }
-      const double2 *wb = (const double2 *)sW + fb * R * L + l;
+      const double2 *wb = (const double2 *)sW + weights(fb) + l;
 #pragma unroll 1
       for (int s = 0; s < n; ++s) {
-        int ff = l + s;
-        if (ff >= n) ff -= n;
-        const int f = fb + ff;
+        const int ff = node(l, s, n), f = fb + (IDLE ? min(ff, Nfq - 1) : ff);
+        const bool on = !IDLE || ff < Nfq;
         const Node B = load<TT>(st, Nq + f);
         pair_means<R, TT>(ahr, ab, alr, alb, B.hr, B.b, B.lr, B.lb, P, rl, pa, ib, pf);
         if (SPLIT) {
@@ -524,16 +527,18 @@ struct VolPairs {
               gm[d] = r ? fma(g2, ah[r][d], gm[d]) : g2 * ah[r][d];
             }
           }
-          double2 *q = (double2 *)acc_f + f;
-          const double2 q0 = q[0], q1 = q[NF];
-          if (DIM == 3) {
-            const double2 q2 = q[2 * NF];
-            q[2 * NF] = make_double2(q2.x + gm[DIM - 1], q2.y + gE);
-          } else {
-            acc_f[4 * NF + f] += gE;
+          if (on) {
+            double2 *q = (double2 *)acc_f + f;
+            const double2 q0 = q[0], q1 = q[NF];
+            if (DIM == 3) {
+              const double2 q2 = q[2 * NF];
+              q[2 * NF] = make_double2(q2.x + gm[DIM - 1], q2.y + gE);
+            } else {
+              acc_f[4 * NF + f] += gE;
+            }
+            q[0] = make_double2(q0.x + g0, q0.y + gp);
+            q[NF] = make_double2(q1.x + gm[0], q1.y + gm[1]);
           }
-          q[0] = make_double2(q0.x + g0, q0.y + gp);
-          q[NF] = make_double2(q1.x + gm[0], q1.y + gm[1]);
         } else {
           double af[Nf], nfv[DIM];
           if (!FACES && CURVED) row_normals(st, ir, f / Nfq, nr);
@@ -563,8 +568,10 @@ struct VolPairs {
 #pragma unroll
             for (int q = 0; q < Nf; ++q) af[q] = r ? fma(w.y, Fr[q], af[q]) : w.y * Fr[q];
           }
+          if (on) {
 #pragma unroll
-          for (int q = 0; q < Nf; ++q) acc_f[q * NF + f] += af[q];
+            for (int q = 0; q < Nf; ++q) acc_f[q * NF + f] += af[q];
+          }
         }
         __syncwarp();
       }
@@ -686,42 +693,53 @@ struct VolPairs {
                                           const uint32_t *__restrict__ mapPq,
                                           const double *__restrict__ uf, const Phys &P) const {
     constexpr int NFG = El::Nfgeo, NPT = (G * NF + TS - 1) / TS;
+    // point u of the thread: its element (in the group) and face node; those
+    // past the group's or the mesh's end repeat a valid one and are not stored
+    auto el = [&](int u) { return min(min((t0 + u * TS) / NF, G - 1), K - 1 - k0 - e0); };
     uint32_t idP[NPT];
 #pragma unroll
-    for (int u = 0; u < NPT; ++u) {
-      const int t = t0 + u * TS, k = k0 + e0 + t / NF;
-      idP[u] = (t < G * NF && k < K) ? mapPq[t % NF + (size_t)k * NF] : 0u;
-    }
+    for (int u = 0; u < NPT; ++u)
+      idP[u] = mapPq[(t0 + u * TS) % NF + (size_t)(k0 + e0 + el(u)) * NF];
+    struct Point {
+      double nJ[DIM], sJ, UM[Nf], UP[Nf];
+    };
+    auto fetch = [&](int u) {
+      Point p;
+      const int f = (t0 + u * TS) % NF;
+      const size_t k = k0 + e0 + el(u);
+      const double *fg = fgeo + k * NF * NFG + f, *um = uf + k * NF * Nf + f, *up = uf + idP[u];
 #pragma unroll
-    for (int u = 0; u < NPT; ++u) {
-      const int t = t0 + u * TS;
-      const int ee = e0 + t / NF, f = t % NF, k = k0 + ee;
-      if (t >= G * NF || k >= K) continue;
-      const size_t idM = f + (size_t)k * NF * Nf;
-      const double *fg = fgeo + (size_t)k * NF * NFG + f;
-      double nJ[DIM];
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) nJ[d] = fg[d * NF];
-      const double sJ = fg[DIM * NF];
-      double UM[Nf], UP[Nf];
+      for (int d = 0; d < DIM; ++d) p.nJ[d] = fg[d * NF];
+      p.sJ = fg[DIM * NF];
 #pragma unroll
       for (int q = 0; q < Nf; ++q) {
-        UM[q] = uf[idM + q * NF];
-        UP[q] = uf[idP[u] + q * NF];
+        p.UM[q] = um[q * NF];
+        p.UP[q] = up[q * NF];
       }
+      return p;
+    };
+    Point p = fetch(0);
+#pragma unroll
+    for (int u = 0; u < NPT; ++u) {
+      Point next;
+      if (u + 1 < NPT) next = fetch(u + 1);  // in flight during this point's arithmetic
+      const int t = t0 + u * TS, ee = e0 + t / NF, f = t % NF;
       double kM, kP, c2M, c2P;
-      const NodeState<DIM> M = node_state_surf<DIM>(UM, 1, P, kM, c2M);
-      const NodeState<DIM> Pp = node_state_surf<DIM>(UP, 1, P, kP, c2P);
+      const NodeState<DIM> M = node_state_surf<DIM>(p.UM, 1, P, kM, c2M);
+      const NodeState<DIM> Pp = node_state_surf<DIM>(p.UP, 1, P, kP, c2P);
       double F[Nf], v[Nf];
-      ecflux_n_nolog<DIM>(M, Pp, nJ, P, F);
+      ecflux_n_nolog<DIM>(M, Pp, p.nJ, P, F);
       const double lamM = fsqrt(kM) + fsqrt(c2M);
       const double lamP = fsqrt(kP) + fsqrt(c2P);
       const double tau = (DIM == 3) ? P.tau : 1.0;
-      const double Lfc = tau * 0.25 * fmax(lamM, lamP) * sJ;
-      face_row(ee, f, v);
+      const double Lfc = tau * 0.25 * fmax(lamM, lamP) * p.sJ;
+      if (t < G * NF && k0 + ee < K) {
+        face_row(ee, f, v);
 #pragma unroll
-      for (int q = 0; q < Nf; ++q) v[q] = v[q] + 0.5 * F[q] - Lfc * (UP[q] - UM[q]);
-      put_row(ee, f, v);
+        for (int q = 0; q < Nf; ++q) v[q] = v[q] + 0.5 * F[q] - Lfc * (p.UP[q] - p.UM[q]);
+        put_row(ee, f, v);
+      }
+      if (u + 1 < NPT) p = next;
     }
   }
 
@@ -731,13 +749,12 @@ struct VolPairs {
     const double *sf = sAcc + e * SA;
 #pragma unroll 1
     for (int fb = T::f0(h); fb < T::f0(h) + T::nf(h); fb += FACES ? Nfq : NF) {
-      const int n = FACES ? Nfq : T::nf(h);
-      const double *wb = sW + 2 * (fb * R * L + l);
+      const int n = steps(h);
+      const double *wb = sW + 2 * (weights(fb) + l);
       for (int s = 0; s < n; ++s) {
-        int ff = l + s;
-        if (ff >= n) ff -= n;
+        const int ff = node(l, s, n);
         double v[Nf];
-        get_row(sf, fb + ff, v);
+        get_row(sf, fb + (IDLE ? min(ff, Nfq - 1) : ff), v);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
           const double w = 2.0 * wb[2 * (s * R + r) * L];
@@ -767,10 +784,10 @@ struct VolPairs {
   __device__ __forceinline__ void group_pairs(double (&acc)[R][Nf], const Phys &P, int e0, int t0,
                                               int ts, Sync gsync) const {
     const double *st = sSt + e * SE;
-    const int range = state_range<NN, L>(l, [&](int n, double &r, double &b) {
+    const int range = state_range<NN, L>(l, [&](int n, int &r, int &b) {
       const double2 a = ((const double2 *)(st + C::oA))[n];
-      r = a.x;
-      b = a.y;
+      r = __double2hiint(a.x);
+      b = __double2hiint(a.y);
     });
     if (range == 0) {
       pairs<0>(acc, P);
@@ -785,12 +802,14 @@ struct VolPairs {
     }
   }
 
-  // warp 1 parks its partial rows in element e's state block (over the
-  // logarithms and densities, [Nf][Nq]; the group's pairs are done)
+  // the warps but the first park their partial rows in element e's state block
+  // ([H - 1][Nf][Nq]; the group's pairs are done).  With two warps they lie over the
+  // logarithms and densities, which face_row does not read; else the face rows
+  // must have been read too
   __device__ __forceinline__ void park_rows(const double (&acc)[R][Nf]) const {
-    static_assert(Nf * Nq <= 4 * NN, "row buffer");
-    double *rowbuf = sSt + e * SE;
-    if (h == 1) {
+    static_assert(Nf * Nq <= 4 * NN && (H - 1) * Nf * Nq <= SE, "row buffer");
+    double *rowbuf = sSt + e * SE + (h - 1) * Nf * Nq;
+    if (h >= 1) {
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const int i = l + L * r;
@@ -801,6 +820,13 @@ struct VolPairs {
       }
     }
   }
+  // field q of row i, summed over the group's warps (the first warp's sum in a)
+  __device__ __forceinline__ double row_sum(double a, int q, int i) const {
+    const double *rowbuf = sSt + e * SE + q * Nq + i;
+#pragma unroll
+    for (int hh = 1; hh < H; ++hh) a += rowbuf[(hh - 1) * Nf * Nq];
+    return a;
+  }
 };
 
 // SURF = false: the volume kernel (euler_vol_*): rhsQ <- the volume rows,
@@ -810,7 +836,7 @@ struct VolPairs {
 // mapPq; Qf is only read, so every element's traces are final) and lifts
 // them into its rows; rhsQ <- the whole right-hand side the surface kernel
 // would leave, rhsQf is not written (fgeo and mapPq unused when false)
-template <int DIM, int N, bool CURVED, int W, bool SURF = false, int RR = 0>
+template <int DIM, int N, bool CURVED, int W, bool SURF = false, int RR = 0, int HH = 0>
 __global__ void __launch_bounds__(32 * W, 1)
 vol_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restrict__ vfgeo,
                  const double *__restrict__ nrJ, const double *__restrict__ nsJ,
@@ -821,11 +847,10 @@ vol_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
                  double *__restrict__ rhsQf, Phys P, const double *__restrict__ fgeo = nullptr,
                  const uint32_t *__restrict__ mapPq = nullptr,
                  const int *__restrict__ blist = nullptr, const int *__restrict__ nblist = nullptr) {
-  using V = VolPairs<DIM, N, CURVED, W, RR>;
+  using V = VolPairs<DIM, N, CURVED, W, RR, HH>;
   constexpr int Nq = V::Nq, NF = V::NF, Nf = V::Nf, R = V::R, L = V::L, E = V::E, H = V::H;
   extern __shared__ double smem[];
   V v(smem);
-  v.load_tables(nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq);
   constexpr bool PRE = V::C::PREFETCH;
   // After the tables, the H warps of an element group touch only their own
   // G elements' shared memory (states, face rows, normals, staged traces),
@@ -850,13 +875,21 @@ vol_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
         double *dst = v.sPre + (size_t)q * G * NF * Nf;
         for (int t = tq; t < n; t += GT) cp_async8(dst + t, src + t);
       } else {
-        for (int t = tq * 16; t < n; t += GT * 16) prefetch_l2(src + t);
+        prefetch_lines(src, n * 8, tq, GT);
       }
       v.fetch_geo(K, kq - q * G, q * G, tq, GT, vgeo);
+      prefetch_lines(rhsQ + (size_t)kq * Nq * Nf, min(K - kq, G) * Nq * Nf * 8, tq, GT);
+      if (CURVED) {
+        prefetch_lines(vgeo + (size_t)kq * Nq * V::NG, min(K - kq, G) * Nq * V::NG * 8, tq, GT);
+        prefetch_lines(vfgeo + (size_t)kq * NF * V::NG, min(K - kq, G) * NF * V::NG * 8, tq, GT);
+      }
+      if (SURF) {
+        prefetch_lines(fgeo + (size_t)kq * NF * V::El::Nfgeo, min(K - kq, G) * NF * V::El::Nfgeo * 8, tq, GT);
+        prefetch_lines(mapPq + (size_t)kq * NF, min(K - kq, G) * NF * 4, tq, GT);
+      }
     }
     cp_async_commit();
   };
-  __syncthreads();  // the tables are shared by every group
   // The work: batches of E elements, all of them or (a work list: the
   // ensemble's active instances) the ascending batch indices blist[0 ..
   // *nblist), each cut into its NG group slices of G elements.  The groups
@@ -875,6 +908,8 @@ vol_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
   };
   const int g0 = q * (int)gridDim.x + (int)blockIdx.x;
   prefetch_group(slice(g0));
+  v.load_tables(nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq);
+  __syncthreads();  // the tables are shared by every group
 
   for (int gi = g0; gi < ns; gi += sstep) {
     const int kg = slice(gi);
@@ -907,20 +942,18 @@ vol_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
         for (int c = 0; c < Nf; ++c) outf[c * NF] = row[c];
       }
     }
+    if (!SURF && H > 2) gsync();  // face rows read: the states become the row buffers
     v.park_rows(acc);
     gsync();
     const int k = k0 + v.e;
-    if (k < K) {
-      const double *rowbuf = v.sSt + v.e * V::SE;
-      if (v.h == 0) {
+    if (k < K && v.h == 0) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int i = v.l + L * r;
-          if (i < Nq) {
-            double *out = rhsQ + (size_t)k * Nq * Nf + i;
+      for (int r = 0; r < R; ++r) {
+        const int i = v.l + L * r;
+        if (i < Nq) {
+          double *out = rhsQ + (size_t)k * Nq * Nf + i;
 #pragma unroll
-            for (int q = 0; q < Nf; ++q) out[q * Nq] = H == 2 ? acc[r][q] + rowbuf[q * Nq + i] : acc[r][q];
-          }
+          for (int q = 0; q < Nf; ++q) out[q * Nq] = v.row_sum(acc[r][q], q, i);
         }
       }
     }
