@@ -63,7 +63,8 @@ int wadg_ctx_set_stream(wadg_ctx *ctx, void *stream);
  * from it; results do not depend on it).  wadg_vol_warps_candidates writes
  * the compiled shapes for the context's degree (at most 3; the first is the
  * default) and returns their number; wadg_ctx_set_vol_warps selects one
- * (0 = the default).  No counterpart in the reference (OCCA's inner-loop
+ * (0 = the default, which on small meshes takes another shape: a warp per face
+ * of an element group).  No counterpart in the reference (OCCA's inner-loop
  * sizes are fixed defines); wadg_app_autotune picks one by timing. */
 int wadg_vol_warps_candidates(const wadg_ctx *ctx, int curved, int *out);
 int wadg_ctx_set_vol_warps(wadg_ctx *ctx, int curved, int warps);

@@ -137,6 +137,29 @@ constexpr int alt_rows() {
   }
 }
 
+// Small meshes take a warp per face (HH = Nfaces, 12 warps) instead of two (or
+// one) per element group: a slice then has half as many pair steps one after another,
+// which is what bounds a kernel of a slice or two per group; fewer groups fit an SM
+// (3 for 6 in 3D, 4 for 6 or 12 in 2D).  So: while the slices are at most
+// one per such group of an SM.  Volume + surface kernel, ms without -> with, by
+// slices per SM: 2D N=3 1.7 .0158 -> .0123, 3.9 .0158 -> .0124, K=32768 (28)
+// .0496 -> .0572; 3D N=2 0.1 .0125 -> .0084, 2.6 .0165 -> .0132, 21 .0745 -> .0777;
+// N=3 0.6 .0162 -> .0111, 2.2 .0222 -> .0186, 5.2 .0312 -> .0339, 42 .200 -> .222;
+// curved N=3 2.2 .0354 -> .0287, 3.5 .0328 -> .0391; curved N=4 2.5 .0528 -> .0401;
+// 2D curved N=4 (faces of 5 nodes, 8 lanes: 3 idle) 3.6 .0244 -> .0166, 14 .0299 -> .0415
+template <int DIM, int N, bool CURVED>
+constexpr int faces_warps() {
+  return VolTile<DIM, N>::H < Elem<DIM, N>::Nfaces ? Elem<DIM, N>::Nfaces : 0;
+}
+template <int DIM, int N, bool CURVED>
+bool small_mesh(const wadg_ctx *c, int K) {
+  if (faces_warps<DIM, N, CURVED>() == 0 || c->vol_warps || c->vol_rows) return false;
+  constexpr int groups = 12 / Elem<DIM, N>::Nfaces;
+  const int slices = (K + VolTile<DIM, N>::G - 1) / VolTile<DIM, N>::G;
+  const int per_sm = (slices + num_sms() - 1) / num_sms();
+  return per_sm <= groups;
+}
+
 // SURF: the volume + surface kernel (rhsQf unused; fgeo, mapPq read)
 template <int DIM, int N, bool CURVED, int W, bool SURF = false, int RR = 0, int HH = 0>
 int launch_vol_pairs_w(const wadg_ctx *c, int K, const double *vgeo, const double *vfgeo,
@@ -168,6 +191,12 @@ int launch_volsurf(const wadg_ctx *c, int K, const double *vgeo, const double *v
                    const double *nsJ, const double *ntJ, const double *Drq, const double *Dsq,
                    const double *Dtq, const double *VqLq, const double *VfPq, const double *Qf,
                    double *rhsQ, const int *blist = nullptr, const int *nb = nullptr) {
+  constexpr int HH = faces_warps<DIM, N, CURVED>();
+  if constexpr (HH > 0)
+    if (small_mesh<DIM, N, CURVED>(c, K))
+      return launch_vol_pairs_w<DIM, N, CURVED, 12, true, 0, HH>(
+          c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, nullptr, fgeo, mapPq,
+          blist, nb);
   constexpr int A0 = alt_rows<DIM, N, CURVED, 0>(), A1 = alt_rows<DIM, N, CURVED, 1>();
   if constexpr (A0 > 0)
     if (c->vol_rows == A0)
@@ -199,6 +228,11 @@ int launch_vol_pairs(const wadg_ctx *c, int K, const double *vgeo, const double 
                      const double *nrJ, const double *nsJ, const double *ntJ, const double *Drq,
                      const double *Dsq, const double *Dtq, const double *VqLq, const double *VfPq,
                      const double *Qf, double *rhsQ, double *rhsQf) {
+  constexpr int HH = faces_warps<DIM, N, CURVED>();
+  if constexpr (HH > 0)
+    if (small_mesh<DIM, N, CURVED>(c, K))
+      return launch_vol_pairs_w<DIM, N, CURVED, 12, false, 0, HH>(
+          c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, rhsQf);
   constexpr int A0 = alt_rows<DIM, N, CURVED, 0>(), A1 = alt_rows<DIM, N, CURVED, 1>();
   if constexpr (A0 > 0)
     if (c->vol_rows == A0)
@@ -319,6 +353,12 @@ int kernel_shape(const wadg_ctx *c, int kernel, int K, int *E, int *grid) {
       if (c->vol_rows == A1) vol_shape<DIM, N, CURVED, alt_warps<DIM, N, CURVED, A1>(), A1>(K, E, grid);
     return WADG_OK;
   }
+  constexpr int HH = faces_warps<DIM, N, CURVED>();
+  if constexpr (HH > 0)
+    if ((kernel == WADG_KERNEL_VOL || kernel == WADG_KERNEL_VOLSURF) && small_mesh<DIM, N, CURVED>(c, K)) {
+      vol_shape<DIM, N, CURVED, 12, 0, HH>(K, E, grid);
+      return WADG_OK;
+    }
   switch (kernel) {
     case WADG_KERNEL_VOL:
       if (W1 && c->vol_warps == W1) vol_shape<DIM, N, CURVED, (W1 ? W1 : 2)>(K, E, grid);

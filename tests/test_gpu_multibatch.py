@@ -220,3 +220,42 @@ def test_adjoint_pair_kernel_over_several_batches(cuda, dim, N, curved):
     _, vjp = torch.func.vjp(T.R, torch.from_numpy(Q).to(dev))
     want = vjp(torch.from_numpy(w).to(dev))[0].cpu().numpy()
     assert rel(gq, want) < 1e-10, rel(gq, want)
+
+
+@pytest.mark.parametrize("dim,N,curved", CASES)
+def test_small_mesh_shape_edges(cuda, dim, N, curved):
+    """Small meshes take another shape of the volume kernels (a warp per face of
+    an element group): the smallest element counts, a partial last slice, the
+    last count that takes it and the first that does not, against the
+    reference's kernels."""
+    ctx = capi.Context(R.load(dim, N))
+    E1 = ctx.shape("volsurf", curved, 1)[0]
+    lo, hi = 1, 1 << 20  # lo takes the small shape, hi does not
+    while hi - lo > 1:
+        mid = (lo + hi) // 2
+        lo, hi = (mid, hi) if ctx.shape("volsurf", curved, mid)[0] == E1 else (lo, mid)
+    assert 300 < lo < 1 << 16 and ctx.shape("vol", curved, lo)[0] == E1 != ctx.shape("vol", curved, hi)[0]
+    geo = build_geometry_gpu(mesh_with_at_least(dim, curved, hi), N)
+    d = Dev(cuda, geo, curved)
+    ref = oracle(geo.ops, curved)
+    st = state(geo, curved, 6)
+    p = lambda s, *names: [s[n].data_ptr() for n in names]
+    geom = ("vgeo", "vfgeo", "nrJ", "nsJ", "ntJ", "Drq", "Dsq", "Dtq", "VqLq", "VfPq")
+    full = {k: v.copy() for k, v in st.items()}
+    ref.vol(geo, full["Qf"], full["rhsQ"], full["rhsQf"])
+    rows, faces = full["rhsQ"].copy(), full["rhsQf"].copy()
+    ref.surf(geo, full["Qf"], full["rhsQf"], full["rhsQ"])
+    for K in (1, 3, lo - 1, lo, hi):
+        s = d.put(st)
+        d.ctx.vol(curved, K, *p(d.g, *geom), *p(s, "Qf", "rhsQ", "rhsQf"))
+        d.sync()
+        h = d.get(s)
+        assert rel(h["rhsQ"][:K], rows[:K]) < RTOL, (K, rel(h["rhsQ"][:K], rows[:K]))
+        assert rel(h["rhsQf"][:K], faces[:K]) < RTOL, (K, rel(h["rhsQf"][:K], faces[:K]))
+        assert np.array_equal(h["rhsQ"][K:], st["rhsQ"][K:]) and (h["rhsQf"][K:] == SENTINEL).all(), K
+        s = d.put(st)
+        d.ctx.volsurf(curved, K, *p(d.g, "vgeo", "vfgeo", "fgeo", "mapPq", *geom[2:]), *p(s, "Qf", "rhsQ"))
+        d.sync()
+        h = d.get(s)
+        assert rel(h["rhsQ"][:K], full["rhsQ"][:K]) < RTOL, (K, rel(h["rhsQ"][:K], full["rhsQ"][:K]))
+        assert np.array_equal(h["rhsQ"][K:], st["rhsQ"][K:]), K
