@@ -100,6 +100,9 @@ int wadg_ctx_sizes(const wadg_ctx *c, int *dim, int *NfqNf) {
   return WADG_OK;
 }
 
+// see wadg_ctx::overlap (the app, while it captures a time step)
+void wadg_ctx_set_overlap(wadg_ctx *c, bool on) { c->overlap = on; }
+
 // the stream a context's kernels run on (used by wadg_noalloc.cu)
 cudaStream_t wadg_ctx_stream(const wadg_ctx *c) { return c ? c->stream : nullptr; }
 

@@ -52,6 +52,12 @@ __device__ __forceinline__ void prefetch_lines(const void *p, int bytes, int t0,
   for (int t = t0 * 128; t < bytes; t += ts * 128) prefetch_l2((const char *)p + t);
 }
 
+// Programmatic dependent launch: let the next kernel of the stream start its
+// preamble, and wait for the previous one to finish (both do nothing in a
+// kernel launched without the attribute)
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
 struct Phys {
   double gamma;
   double gm1;     // gamma - 1

@@ -51,6 +51,8 @@ surf_mma_kernel(int K, const double *__restrict__ fgeo, const uint32_t *__restri
   const int ne = min(EW, K - k0);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
+  pdl_trigger();
+  pdl_wait();
   // ---- surface flux at the group's face points -> SF
   for (int t = threadIdx.x; t < EW * NF; t += C::threads) {
     const int e = t / NF, j = t - e * NF;

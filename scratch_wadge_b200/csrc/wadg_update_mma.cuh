@@ -332,6 +332,8 @@ update_mma_kernel(int K, const double *__restrict__ Jq, const double *__restrict
     Y[Nq * LD + t] = 0.0;
   }
 
+  pdl_trigger();
+  pdl_wait();
   // the groups to run: all of them, or (a work list: the ensemble's active
   // instances) the group indices blist[0 .. *nblist); dtK: a step per element
   const int ngroups = blist ? *nblist : (K + EW - 1) / EW;

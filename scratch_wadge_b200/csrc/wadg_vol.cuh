@@ -907,8 +907,15 @@ vol_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
     return (blist ? blist[cb] : cb) * E + (g - cb * NG) * G;
   };
   const int g0 = q * (int)gridDim.x + (int)blockIdx.x;
-  prefetch_group(slice(g0));
-  v.load_tables(nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq);
+  if (HH > 0) {  // launched to overlap the previous kernel's end on the smallest meshes
+    pdl_trigger();
+    v.load_tables(nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq);  // no kernel's output
+    pdl_wait();
+    prefetch_group(slice(g0));
+  } else {
+    prefetch_group(slice(g0));
+    v.load_tables(nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq);
+  }
   __syncthreads();  // the tables are shared by every group
 
   for (int gi = g0; gi < ns; gi += sstep) {
