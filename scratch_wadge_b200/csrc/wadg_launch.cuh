@@ -408,20 +408,39 @@ int kernel_shape(const wadg_ctx *c, int kernel, int K, int *E, int *grid) {
   return fail(WADG_ERR_INVALID, "unknown kernel %d", kernel);
 }
 
+// Meshes of few groups take the wide shape: up to one group per SM in 3D, three
+// in 2D.  Update kernel, us, default -> wide, by groups per SM: 3D N=2 0.1 5.5 ->
+// 4.0, 2.6 6.5 -> 7.3; N=3 0.3 6.9 -> 5.4, 1.1 7.9 -> 8.9; curved N=4 0.6 13.8 -> 11.6,
+// 1.7 20.0 -> 21.4; 2D N=3 1.7 4.6 -> 4.2, 2.7 5.0 -> 4.4, 6.9 7.6 -> 7.9
+template <int DIM, int N, bool CURVED>
+bool wide_update(int K) {
+  return K <= (DIM == 3 ? 1 : 3) * num_sms() * UpdMmaCfg<DIM, N, CURVED>::EW;
+}
+
+template <int DIM, int N, bool CURVED, bool WIDE>
+int launch_update_w(const wadg_ctx *c, int K, int grid, const double *Jq, const double *VqPq,
+                    const double *VfPq, double fa, double fb, double fdt, double *rhsQ, double *resQ,
+                    double *Q, double *Qf, const double *dtK, const int *glist, const int *ng) {
+  using C = UpdMmaCfg<DIM, N, CURVED, WIDE>;
+  static_assert(C::smem <= 227 * 1024, "update kernel does not fit in shared memory");
+  if (int r = launch(c, overlaps<DIM, N>(c, K), update_mma_kernel<DIM, N, CURVED, WIDE>, grid, C::threads,
+                     C::smem, K, Jq, VqPq, VfPq, fa, fb, fdt, rhsQ, resQ, Q, Qf, c->phys, dtK, glist, ng))
+    return r;
+  return after_launch("update kernel");
+}
+
 template <int DIM, int N, bool CURVED>
 int launch_update(const wadg_ctx *c, int K, const double *Jq, const double *VqPq,
                   const double *VfPq, double fa, double fb, double fdt, double *rhsQ,
                   double *resQ, double *Q, double *Qf, const double *dtK = nullptr,
                   const int *glist = nullptr, const int *ng = nullptr) {
-  using C = UpdMmaCfg<DIM, N, CURVED>;
-  static_assert(C::smem <= 227 * 1024, "update kernel does not fit in shared memory");
-  auto kern = update_mma_kernel<DIM, N, CURVED>;
   int grid = 0;
   if (int r = update_grid<DIM, N, CURVED>(K, &grid)) return r;
-  if (int r = launch(c, overlaps<DIM, N>(c, K), kern, grid, C::threads, C::smem, K, Jq, VqPq, VfPq, fa, fb, fdt, rhsQ, resQ, Q,
-                     Qf, c->phys, dtK, glist, ng))
-    return r;
-  return after_launch("update kernel");
+  if (wide_update<DIM, N, CURVED>(K))
+    return launch_update_w<DIM, N, CURVED, true>(c, K, grid, Jq, VqPq, VfPq, fa, fb, fdt, rhsQ, resQ, Q,
+                                                 Qf, dtK, glist, ng);
+  return launch_update_w<DIM, N, CURVED, false>(c, K, grid, Jq, VqPq, VfPq, fa, fb, fdt, rhsQ, resQ, Q,
+                                                Qf, dtK, glist, ng);
 }
 
 // every launch of one (dim, N, curved), defined in wadg_k<dim><N>.cu

@@ -41,7 +41,10 @@ __device__ __forceinline__ void dmma884(double &d0, double &d1, double a, double
 
 constexpr int mma_ld(int c) { return (c % 16 == 4 || c % 16 == 12) ? c : mma_ld(c + 1); }
 
-template <int DIM, int N, bool CURVED>
+// WIDE: a warp per m-tile of the output projection too, for meshes of a group or
+// two per SM, where a kernel takes as long as one group does (three m-tiles one after
+// another in a warp at 3D N=3)
+template <int DIM, int N, bool CURVED, bool WIDE = false>
 struct UpdMmaCfg {
   using El = Elem<DIM, N>;
   static constexpr int Nq = El::Nq, NF = El::NfqNf, Nf = El::Nfields;
@@ -54,7 +57,7 @@ struct UpdMmaCfg {
   static constexpr int BUF = KP * LD;               // one buffer
   // one CTA works on one group at a time, one warp per m-tile of the Nq x Nq
   // products (the output projection's MO m-tiles go round-robin)
-  static constexpr int WARPS = MQ < 2 ? 2 : (MQ > 6 ? 6 : MQ);
+  static constexpr int WARPS = WIDE ? MO : MQ < 2 ? 2 : (MQ > 6 ? 6 : MQ);
   static constexpr int threads = 32 * WARPS;
   static constexpr size_t smem = sizeof(double) * 2 * BUF;
   // register cap from the launch bounds.  Up to 3 warps per CTA, 5 resident
@@ -63,7 +66,7 @@ struct UpdMmaCfg {
   // registers).  At 6 warps (N=4 in 3D), 5 CTAs cap the registers at 64 and
   // spill: 3 CTAs measured best (curved N=4: 0.0885 ms vs 0.0965 at 5,
   // 0.100 at 2, 0.091 at 4)
-  static constexpr int min_ctas = WARPS >= 6 ? 3 : 5;
+  static constexpr int min_ctas = WIDE ? 1 : WARPS >= 6 ? 3 : 5;
 };
 
 // A fragments of rows [8 mt, 8 mt + 8) of an operator stored column-major
@@ -313,14 +316,14 @@ __device__ __forceinline__ void stage_rhs(const double *rhs, int k0, int ne, dou
   }
 }
 
-template <int DIM, int N, bool CURVED>
-__global__ void __launch_bounds__(UpdMmaCfg<DIM, N, CURVED>::threads, UpdMmaCfg<DIM, N, CURVED>::min_ctas)
+template <int DIM, int N, bool CURVED, bool WIDE = false>
+__global__ void __launch_bounds__(UpdMmaCfg<DIM, N, CURVED, WIDE>::threads, UpdMmaCfg<DIM, N, CURVED, WIDE>::min_ctas)
 update_mma_kernel(int K, const double *__restrict__ Jq, const double *__restrict__ VqPq,
                   const double *__restrict__ VfPq, double fa, double fb, double fdt,
                   double *__restrict__ rhsQ, double *__restrict__ resQ, double *__restrict__ Q,
                   double *__restrict__ Qf, Phys P, const double *__restrict__ dtK = nullptr,
                   const int *__restrict__ blist = nullptr, const int *__restrict__ nblist = nullptr) {
-  using C = UpdMmaCfg<DIM, N, CURVED>;
+  using C = UpdMmaCfg<DIM, N, CURVED, WIDE>;
   constexpr int Nq = C::Nq, Nf = C::Nf, EW = C::EW, KP = C::KP, LD = C::LD, MQ = C::MQ;
   extern __shared__ double smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -346,7 +349,7 @@ update_mma_kernel(int K, const double *__restrict__ Jq, const double *__restrict
       if (warp < MQ) load_lsrk<Nq, Nf>(resQ, Q, Jq, k0, ne, warp, lane, res0, q0, Jv);
     });
     __syncthreads();
-    update_group<DIM, N, CURVED>(k0, ne, warp, lane, X, Y, Jq, VqPq, VfPq, fa, fb, fdt, resQ, Q,
+    update_group<DIM, N, CURVED, C::WARPS>(k0, ne, warp, lane, X, Y, Jq, VqPq, VfPq, fa, fb, fdt, resQ, Q,
                                  rhsQ, Qf, P, res0, q0, Jv, dtK);
   }
 }

@@ -259,3 +259,29 @@ def test_small_mesh_shape_edges(cuda, dim, N, curved):
         h = d.get(s)
         assert rel(h["rhsQ"][:K], full["rhsQ"][:K]) < RTOL, (K, rel(h["rhsQ"][:K], full["rhsQ"][:K]))
         assert np.array_equal(h["rhsQ"][K:], st["rhsQ"][K:]), K
+
+
+@pytest.mark.parametrize("dim,N,curved", CASES)
+def test_update_shape_edges(cuda, dim, N, curved):
+    """The update kernel's two shapes (a warp per m-tile of the output projection
+    on meshes of few groups): a single element, a partial group, and the last
+    element count of the wide shape and the first past it, against the
+    reference's kernel."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    last = (1 if dim == 3 else 3) * sms * 8
+    geo = build_geometry_gpu(mesh_with_at_least(dim, curved, last + 1), N)
+    d = Dev(cuda, geo, curved)
+    st = state(geo, curved, 8)
+    st["rhsQ"] = 1e-3 * st["rhsQ"]
+    dt = IC.time_step(geo, 0.1, N, nsteps=1, wave_speed=IC.max_wave_speed(st["Q"]))[0]
+    for K in (1, 9, last, last + 1):
+        s = d.put(st)
+        d.ctx.update(curved, K, *[d.g[n].data_ptr() for n in ("Jq", "VqPq", "VfPq")], IC.RK4A[1],
+                     IC.RK4B[1], dt, *[s[n].data_ptr() for n in ("rhsQ", "resQ", "Q", "Qf")])
+        d.sync()
+        h = d.get(s)
+        a = _first(st, K)
+        oracle(geo.ops, curved).update(geo, IC.RK4A[1], IC.RK4B[1], dt, a["rhsQ"], a["resQ"], a["Q"], a["Qf"])
+        for k in ("Q", "rhsQ", "Qf", "resQ"):
+            assert np.isfinite(a[k]).all() and rel(h[k][:K], a[k]) < RTOL, (K, k, rel(h[k][:K], a[k]))
+            assert np.array_equal(h[k][K:], st[k][K:]), (K, k)
