@@ -58,6 +58,10 @@ struct UpdMmaCfg {
   // one CTA works on one group at a time, one warp per m-tile of the Nq x Nq
   // products (the output projection's MO m-tiles go round-robin)
   static constexpr int WARPS = WIDE ? MO : MQ < 2 ? 2 : (MQ > 6 ? 6 : MQ);
+  // a warp's m-tiles of the output projection share the fragments of its operand
+  // where it has three of them (3D N=2, 3): 0.0537 -> 0.0499 ms at N=3, K=24576;
+  // the shorter or longer cases (2D; 3D N=4 with its 11 k-steps) lose 1-4 %
+  static constexpr bool SHARE = DIM == 3 && (N == 2 || N == 3) && !WIDE;
   static constexpr int threads = 32 * WARPS;
   static constexpr size_t smem = sizeof(double) * 2 * BUF;
   // register cap from the launch bounds.  Up to 3 warps per CTA, 5 resident
@@ -66,7 +70,8 @@ struct UpdMmaCfg {
   // registers).  At 6 warps (N=4 in 3D), 5 CTAs cap the registers at 64 and
   // spill: 3 CTAs measured best (curved N=4: 0.0885 ms vs 0.0965 at 5,
   // 0.100 at 2, 0.091 at 4)
-  static constexpr int min_ctas = WIDE ? 1 : WARPS >= 6 ? 3 : 5;
+  // At 3D N=2 (2 warps) 8 CTAs: 0.0111 -> 0.0092 ms at K=7986, 10 0.0096
+  static constexpr int min_ctas = WIDE ? 1 : WARPS >= 6 ? 3 : DIM == 3 && N == 2 ? 8 : 5;
 };
 
 // A fragments of rows [8 mt, 8 mt + 8) of an operator stored column-major
@@ -82,24 +87,12 @@ __device__ __forceinline__ void load_afrag(const double *__restrict__ Op, int ld
   }
 }
 
-// the stacked operator [VfPq; VqPq] (NF + Nq rows)
-template <int KS, int Nq, int NF>
-__device__ __forceinline__ void load_afrag_out(const double *__restrict__ VfPq,
-                                               const double *__restrict__ VqPq, int mt, int lane,
-                                               double *a) {
-  const int m = mt * 8 + (lane >> 2);
-#pragma unroll
-  for (int ks = 0; ks < KS; ++ks) {
-    const int k = ks * 4 + (lane & 3);
-    double v = 0.0;
-    if (k < Nq) {
-      if (m < NF)
-        v = __ldg(VfPq + m + (size_t)k * NF);
-      else if (m < NF + Nq)
-        v = __ldg(VqPq + (m - NF) + (size_t)k * Nq);
-    }
-    a[ks] = v;
-  }
+// entry (m, k) of the stacked operator [VfPq; VqPq] (NF + Nq rows); zero outside
+template <int Nq, int NF>
+__device__ __forceinline__ double afrag_out(const double *__restrict__ VfPq,
+                                            const double *__restrict__ VqPq, int m, int k) {
+  if (k >= Nq || m >= NF + Nq) return 0.0;
+  return m < NF ? __ldg(VfPq + m + (size_t)k * NF) : __ldg(VqPq + (m - NF) + (size_t)k * Nq);
 }
 
 // D[f][i] = sum_k A(m, k) X(k, f*8 + e), m = 8 mt + lane/4, e = 2 (lane%4) + i
@@ -264,24 +257,53 @@ __device__ __forceinline__ void update_group(
   }
 
   // ---- Qf = U(VfPq v), rhsQ = U(VqPq v)
-  for (int mt = warp; mt < MO; mt += W) {
-    load_afrag_out<KS, Nq, NF>(VfPq, VqPq, mt, lane, a);
-    mtile_gemm<KS, Nf, LD>(a, Xo, lane, D);
-    const int m = mt * 8 + (lane >> 2);
-    if (m >= NF + Nq) continue;
+  auto put = [&](int m, const double (&Dm)[Nf][2]) {
+    if (m >= NF + Nq) return;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       if (!ev[i]) continue;
       const int e = 2 * (lane & 3) + i;
       double V[Nf], U[Nf];
 #pragma unroll
-      for (int f = 0; f < Nf; ++f) V[f] = D[f][i];
+      for (int f = 0; f < Nf; ++f) V[f] = Dm[f][i];
       UV<DIM>(V, U, P);
       double *out = m < NF ? Qf_out + (size_t)(k0 + e) * NF * Nf + m
                            : rhsQ_out + (size_t)(k0 + e) * Nq * Nf + (m - NF);
       const int ld = m < NF ? NF : Nq;
 #pragma unroll
       for (int f = 0; f < Nf; ++f) out[f * ld] = U[f];
+    }
+  };
+  if constexpr (C::SHARE && UW == C::WARPS) {
+    constexpr int MB = (MO + W - 1) / W;
+    double Db[MB][Nf][2];
+#pragma unroll
+    for (int j = 0; j < MB; ++j)
+#pragma unroll
+      for (int f = 0; f < Nf; ++f) Db[j][f][0] = Db[j][f][1] = 0.0;
+    const double *xb = Xo + (lane & 3) * LD + (lane >> 2);
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+      double b[Nf], ab[MB];
+#pragma unroll
+      for (int j = 0; j < MB; ++j)
+        ab[j] = afrag_out<Nq, NF>(VfPq, VqPq, (warp + j * W) * 8 + (lane >> 2), ks * 4 + (lane & 3));
+#pragma unroll
+      for (int f = 0; f < Nf; ++f) b[f] = xb[ks * 4 * LD + f * 8];
+#pragma unroll
+      for (int j = 0; j < MB; ++j)
+#pragma unroll
+        for (int f = 0; f < Nf; ++f) dmma884(Db[j][f][0], Db[j][f][1], ab[j], b[f]);
+    }
+#pragma unroll
+    for (int j = 0; j < MB; ++j) put((warp + j * W) * 8 + (lane >> 2), Db[j]);
+  } else {
+    for (int mt = warp; mt < MO; mt += W) {
+#pragma unroll
+      for (int ks = 0; ks < KS; ++ks)
+        a[ks] = afrag_out<Nq, NF>(VfPq, VqPq, mt * 8 + (lane >> 2), ks * 4 + (lane & 3));
+      mtile_gemm<KS, Nf, LD>(a, Xo, lane, D);
+      put(mt * 8 + (lane >> 2), D);
     }
   }
 }
