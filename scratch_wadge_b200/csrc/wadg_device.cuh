@@ -347,18 +347,26 @@ __device__ __forceinline__ void pair_means(const double (&ahr)[R], const double 
 
 // Two-point flux F_S(a, b).n for states without precomputed logarithms (surface
 // traces): beyond the series range the log-mean evaluates log(a/b) itself, as
-// the reference does.
-template <int DIM>
+// the reference does.  WARP: called by all 32 lanes, which take the short
+// polynomials where all their pairs allow it (traces of a smooth flow differ
+// little across a face)
+template <int DIM, bool WARP = false>
 __device__ __forceinline__ void ecflux_n_nolog(const NodeState<DIM> &a, const NodeState<DIM> &b,
                                                const double *n, const Phys &P, double *F) {
-  const double sr = a.rho + b.rho, dr = a.rho - b.rho;
+  const double hs = 0.5 * (a.rho + b.rho), dr = a.rho - b.rho;
   const double sb = a.beta + b.beta, db = a.beta - b.beta;
-  const double isr = rcp(sr), isb = rcp(sb);
-  const double fr = dr * isr, fb = db * isb;
+  const double isr = rcp(hs), isb = rcp(sb);
+  const double fr = 0.5 * dr * isr, fb = db * isb;
   const double ur = fr * fr, ub = fb * fb;
-  const double rl = (ur < logmean_u(2)) ? 0.5 * sr * polyG<2>(ur) : dr / log(a.rho / b.rho);
-  const double ibl = (ub < logmean_u(2)) ? 2.0 * isb * polyF<2>(ub) : log(a.beta / b.beta) / db;
-  const double pa = 0.5 * sr * isb;
+  double rl, ib;  // L(rho), 1/(2(gamma-1) L(beta))
+  if (WARP && __all_sync(0xffffffffu, fmax(ur, ub) < logmean_u(0))) {
+    rl = hs * polyG<0>(ur);
+    ib = isb * fma(fma(P.f2, ub, P.f1), ub, P.igm1);
+  } else {
+    rl = ur < logmean_u(2) ? hs * polyG<2>(ur) : dr / log(a.rho / b.rho);
+    ib = ub < logmean_u(2) ? isb * P.igm1 * polyF<2>(ub) : P.cbeta * (log(a.beta / b.beta) / db);
+  }
+  const double pa = hs * isb;
   double ub2[DIM], un = 0.0, vv = 0.0;
 #pragma unroll
   for (int d = 0; d < DIM; ++d) {
@@ -366,7 +374,7 @@ __device__ __forceinline__ void ecflux_n_nolog(const NodeState<DIM> &a, const No
     un = fma(ub2[d], n[d], un);
     vv = fma(a.vel[d], b.vel[d], vv);
   }
-  const double f4 = fma(rl, fma(ibl, P.cbeta, 0.5 * vv), pa);
+  const double f4 = fma(rl, fma(0.5, vv, ib), pa);
   const double F0 = rl * un;
   F[0] = F0;
 #pragma unroll
@@ -374,18 +382,17 @@ __device__ __forceinline__ void ecflux_n_nolog(const NodeState<DIM> &a, const No
   F[DIM + 1] = f4 * un;
 }
 
-// sqrt(x) for x >= 0 (0 for x <= 0): the reciprocal square root estimate
-// rsqrt.approx.f64 refined by two Newton-Raphson steps on y^-2 = x, then one
-// Newton step on s^2 = x for s = x y; a few ulp, for the surface kernels'
+// sqrt(x) for x >= 0 (0 for x <= 0): one third-order step on the reciprocal
+// square root estimate y0: with s0 = x y0 and e = 1 - s0 y0, sqrt(x) = s0 (1 -
+// e)^(-1/2) = s0 (1 + e/2 + 3 e^2/8) + O(e^3), |e| < 1.9e-6 (measured
+// over [1, 4)): rounding error, in five operations.  For the surface kernels'
 // wave speeds (which only enter the penalty's max)
 __device__ __forceinline__ double fsqrt(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  y = y * fma(-0.5 * x * y, y, 1.5);
-  y = y * fma(-0.5 * x * y, y, 1.5);
-  double s = x * y;
-  s = fma(0.5 * y, fma(-s, s, x), s);
-  return x > 0.0 ? s : 0.0;
+  const double s = x * y;
+  const double e = fma(-s, y, 1.0);
+  return x > 0.0 ? fma(s * e, fma(e, 0.375, 0.5), s) : 0.0;
 }
 
 // node state of a conservative trace without the logarithms (for

@@ -644,7 +644,8 @@ struct VolPairs {
     v[DIM + 1] = gE;
   }
 
-  // a face row back into its slots, for the lift
+  // a face row back into its slots, for the lift (twice the row: the lift's
+  // weights 1/2 VqLq are the pair phase's)
   __device__ __forceinline__ void put_row(int ee, int f, const double (&v)[Nf]) const {
     double *acc_f = sAcc + ee * SA;
     if (SPLIT) {
@@ -728,7 +729,7 @@ struct VolPairs {
       const NodeState<DIM> M = node_state_surf<DIM>(p.UM, 1, P, kM, c2M);
       const NodeState<DIM> Pp = node_state_surf<DIM>(p.UP, 1, P, kP, c2P);
       double F[Nf], v[Nf];
-      ecflux_n_nolog<DIM>(M, Pp, p.nJ, P, F);
+      ecflux_n_nolog<DIM, true>(M, Pp, p.nJ, P, F);
       const double lamM = fsqrt(kM) + fsqrt(c2M);
       const double lamP = fsqrt(kP) + fsqrt(c2P);
       const double tau = (DIM == 3) ? P.tau : 1.0;
@@ -736,14 +737,14 @@ struct VolPairs {
       if (t < G * NF && k0 + ee < K) {
         face_row(ee, f, v);
 #pragma unroll
-        for (int q = 0; q < Nf; ++q) v[q] = v[q] + 0.5 * F[q] - Lfc * (p.UP[q] - p.UM[q]);
+        for (int q = 0; q < Nf; ++q) v[q] = fma(-2.0 * Lfc, p.UP[q] - p.UM[q], fma(2.0, v[q], F[q]));
         put_row(ee, f, v);
       }
       if (u + 1 < NPT) p = next;
     }
   }
 
-  // lift: rows += VqLq sf on the rotated weights (VqLq = 2 W1), the warps of
+  // lift: rows += (1/2 VqLq) (2 sf) on the rotated weights, the warps of
   // the group splitting the face nodes as in the pair phase
   __device__ __forceinline__ void lift(double (&acc)[R][Nf]) const {
     const double *sf = sAcc + e * SA;
@@ -757,7 +758,7 @@ struct VolPairs {
         get_row(sf, fb + (IDLE ? min(ff, Nfq - 1) : ff), v);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-          const double w = 2.0 * wb[2 * (s * R + r) * L];
+          const double w = wb[2 * (s * R + r) * L];
 #pragma unroll
           for (int q = 0; q < Nf; ++q) acc[r][q] = fma(w, v[q], acc[r][q]);
         }
