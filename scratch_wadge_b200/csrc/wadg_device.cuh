@@ -185,6 +185,19 @@ __device__ __forceinline__ NodeState<DIM> node_state(const double *q, const Phys
   return s;
 }
 
+// sqrt(x) for x >= 0 (0 for x <= 0): one third-order step on the reciprocal
+// square root estimate y0: with s0 = x y0 and e = 1 - s0 y0, sqrt(x) = s0 (1 -
+// e)^(-1/2) = s0 (1 + e/2 + 3 e^2/8) + O(e^3), |e| < 1.9e-6 (measured
+// over [1, 4)): rounding error, in five operations.  For the surface kernels'
+// wave speeds (which only enter the penalty's max)
+__device__ __forceinline__ double fsqrt(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double s = x * y;
+  const double e = fma(-s, y, 1.0);
+  return x > 0.0 ? fma(s * e, fma(e, 0.375, 0.5), s) : 0.0;
+}
+
 // conservative -> entropy variables (Euler3Daffine.okl:73-93 / Euler2D.okl:69-87)
 template <int DIM>
 __device__ __forceinline__ void VU(const double *U, double *V, const Phys &P) {
@@ -219,7 +232,7 @@ __device__ __forceinline__ void UV(const double *V, double *U, const Phys &P) {
   double rhoe;
   if (P.gamma == 1.4) {
     const double mv = -Vl;
-    rhoe = exp((P.lgm1 - sV) * P.igm1) * rcp(mv * mv * mv * sqrt(mv));
+    rhoe = exp((P.lgm1 - sV) * P.igm1) * rcp(mv * mv * mv * fsqrt(mv));
   } else {
     rhoe = exp((P.lgm1 - P.gamma * log(-Vl) - sV) * P.igm1);
   }
@@ -380,19 +393,6 @@ __device__ __forceinline__ void ecflux_n_nolog(const NodeState<DIM> &a, const No
 #pragma unroll
   for (int d = 0; d < DIM; ++d) F[1 + d] = fma(F0, ub2[d], pa * n[d]);
   F[DIM + 1] = f4 * un;
-}
-
-// sqrt(x) for x >= 0 (0 for x <= 0): one third-order step on the reciprocal
-// square root estimate y0: with s0 = x y0 and e = 1 - s0 y0, sqrt(x) = s0 (1 -
-// e)^(-1/2) = s0 (1 + e/2 + 3 e^2/8) + O(e^3), |e| < 1.9e-6 (measured
-// over [1, 4)): rounding error, in five operations.  For the surface kernels'
-// wave speeds (which only enter the penalty's max)
-__device__ __forceinline__ double fsqrt(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double s = x * y;
-  const double e = fma(-s, y, 1.0);
-  return x > 0.0 ? fma(s * e, fma(e, 0.375, 0.5), s) : 0.0;
 }
 
 // node state of a conservative trace without the logarithms (for
