@@ -86,7 +86,11 @@ constexpr int adjW() {
   constexpr int H = C1::H;
   constexpr size_t per_warp = sizeof(double) * (size_t)C1::per_elem * VolTile<DIM, N>::G / H;
   constexpr size_t w = (227 * 1024 - C1::fixed) / per_warp;
-  constexpr int wc = w >= 12 ? 12 : (int)w;
+  // 12 (168 registers per thread) or at most 8 (255): 10 would leave them 168 for
+  // less work, and three rows per lane in 3D need about 250.  Below 8, six warps
+  // where they hold 12 elements, else 4 (curved 3D N=4: six were not measured)
+  constexpr int cap = DIM == 3 && VolTile<DIM, N>::R >= 3 ? 8 : 12;
+  constexpr int wc = w >= 12 && cap == 12 ? 12 : w >= 8 ? 8 : w >= 6 && VolTile<DIM, N>::G >= 4 ? 6 : w >= 4 ? 4 : (int)w;
   return wc < H ? H : (wc / H) * H;
 }
 

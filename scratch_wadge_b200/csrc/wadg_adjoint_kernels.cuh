@@ -36,127 +36,190 @@
 
 namespace wadg {
 
-// node state of the pair VJP: NodeState plus 1/rho and 1/beta
+// node state of the node-level adjoints: NodeState plus 1/rho and 1/beta
 template <int DIM> struct AdjNode {
-  double rho, vel[DIM], beta, lrho, lbeta, irho, ibeta;
+  double rho, vel[DIM], beta, irho, ibeta;
 };
 
-// F(u) = sum_{k<=8} u^k/(2k+1) and dF/du
-__device__ __forceinline__ void polyF_d(double u, double &F, double &dF) {
-  const double c[9] = {1.0, 1.0 / 3.0, 1.0 / 5.0, 1.0 / 7.0, 1.0 / 9.0,
-                       1.0 / 11.0, 1.0 / 13.0, 1.0 / 15.0, 1.0 / 17.0};
-  F = c[8];
-  dF = 0.0;
-#pragma unroll
-  for (int k = 7; k >= 0; --k) {
-    dF = fma(dF, u, F);
-    F = fma(F, u, c[k]);
+// 2 F'(u) and 2 G'(u) of the log-mean's F and G = 1/F over [0, logmean_u(T)]
+// (Chebyshev interpolants like polyF and polyG; relative error below 2e-16,
+// for 2 G' at T = 2 2e-15 -- they enter multiplied by f, |f| < 0.25)
+template <int T> __device__ __forceinline__ double poly2dF(double u) {
+  if (T == 0) return fma(fma(0.8571601907354554, u, 0.7999999999154984), u, 0.6666666666666667);
+  double p;
+  if (T == 1) {
+    p = 0.9137215016503201;
+    p = fma(p, u, 0.8888807768596552);
+    p = fma(p, u, 0.8571428629398847);
+    p = fma(p, u, 0.7999999999985504);
+  } else {
+    p = 1.2506608372608468;
+    p = fma(p, u, 0.9052414855673793);
+    p = fma(p, u, 0.9355690465677214);
+    p = fma(p, u, 0.9229967150047704);
+    p = fma(p, u, 0.9090925902016338);
+    p = fma(p, u, 0.8888888691610057);
+    p = fma(p, u, 0.8571428572585671);
+    p = fma(p, u, 0.7999999999997391);
   }
+  return fma(p, u, 0.6666666666666667);
 }
-// G(u) = 1/F(u) to degree 8 (the coefficients of polyG) and dG/du
-__device__ __forceinline__ void polyG_d(double u, double &G, double &dG) {
-  const double c[9] = {1.0, -1.0 / 3.0, -4.0 / 45.0, -44.0 / 945.0, -428.0 / 14175.0,
-                       -10196.0 / 467775.0, -10719068.0 / 638512875.0,
-                       -25865068.0 / 1915538625.0, -5472607916.0 / 488462349375.0};
-  G = c[8];
-  dG = 0.0;
-#pragma unroll
-  for (int k = 7; k >= 0; --k) {
-    dG = fma(dG, u, G);
-    G = fma(G, u, c[k]);
+template <int T> __device__ __forceinline__ double poly2dG(double u) {
+  if (T == 0) return fma(fma(-0.27936978969179216, u, -0.3555555555325926), u, -0.6666666666666666);
+  double p;
+  if (T == 1) {
+    p = -0.21897837304155307;
+    p = fma(p, u, -0.24155025841658195);
+    p = fma(p, u, -0.2793650806297747);
+    p = fma(p, u, -0.3555555555552393);
+    return fma(p, u, -0.6666666666666666);
   }
+  p = -0.22666051739367454;
+  p = fma(p, u, -0.1842050736194697);
+  p = fma(p, u, -0.2017014006762885);
+  p = fma(p, u, -0.21796089954717837);
+  p = fma(p, u, -0.24155213809387097);
+  p = fma(p, u, -0.2793650785373233);
+  p = fma(p, u, -0.355555555557926);
+  return fma(p, u, -0.6666666666666655);
 }
+
+template <int V> struct IntTag {
+  static constexpr int value = V;
+};
 
 // Vector-Jacobian product of the contracted two-point flux F_S(a, b).n
-// (ecflux_n; Euler3Daffine.okl:107-148, Euler2D.okl:139-161) with the
-// adjoint c of its Nfields components, split into the part that depends on
-// the two states only (FluxCore: the means and their partial derivatives)
-// and a reverse sweep per (n, c) that adds the adjoints of a's and b's
-// primitive states (rho, velocity, beta) to ba and bb.
+// (Euler3Daffine.okl:107-148, Euler2D.okl:139-161) with the
+// adjoint c of its Nfields components: adds the adjoints of a's and b's
+// states to ba and bb.
 //
-// Log-mean derivatives (L(a,b) = (a-b)/(log a - log b), s = a+b, f = (a-b)/s,
-// u = f^2):
-//   log form:    dL/da = (1 - L/a)/(log a - log b), dL/db = (L/b - 1)/(log a - log b)
-//   series form: L = s/2 G(u): dL/da = G/2 + G'(u) f (1-f), dL/db = G/2 - G' f (1+f)
-// and for 1/L (the inverse-temperature mean, 1/L = 2F(u)/s):
-//   log form:    d(1/L)/da = (1/a - 1/L)/(a-b), d(1/L)/db = (1/L - 1/b)/(a-b)
-//   series form: d(1/L)/da = 2/s^2 (-F + 2F' f(1-f)), d(1/L)/db = 2/s^2 (-F - 2F' f(1+f))
-// with the same branch switch (u < 1e-2) as the forward flux.
+// Pair loops (pair_vjp): the states are hr = rho/2, h = u/2 and beta, the
+// adjoints those of (hr, h, beta).  With sr = hr_a + hr_b, fr = (hr_a - hr_b)/sr, ur = fr^2,
+// G(ur) = 1/F(ur), and sb, fb, ub of the betas: rl = sr G, pa = sr/sb, ubar = h_a + h_b,
+//   ib = 1/(2(gamma-1) L(beta)) = m F(ub), m = 1/((gamma-1) sb),
+//   F0 = rl un, Fm = F0 ubar + pa n, FE = (rl (ib + 2 h_a.h_b) + pa) un.
+// Derivatives of the log-means, T = 2 G' fr and S = 2 F' fb:
+//   d rl/d hr_a = G - T fr + T,  d rl/d hr_b = G - T fr - T,
+//   d ib/d beta_a = m/sb (-F - S fb + S),  d ib/d beta_b = m/sb (-F - S fb - S).
+// Log form (T = 3, u beyond the polynomials; rho = 2 hr):
+//   d L/d rho_a = (1 - L/rho_a)/(log rho_a - log rho_b), d L/d rho_b = (L/rho_b - 1)/(...),
+//   d ib/d beta_a = (c/beta_a - ib)/(beta_a - beta_b), d ib/d beta_b = (ib - c/beta_b)/(...),
+// c = 1/(2(gamma-1)).  TT: the range of the states (state_range).  88 FP64
+// operations per pair at TT = 0 beside its direction and seed, where (rho, u,
+// beta) and one branch for u < 4e-6 took 106; the FP64 pipe bounds the kernel
+// (59 % active at 8 warps).  With the logarithms only where a group needs them:
+// gradient of 20 steps, K=3072 N=3, 19.4 -> 16.5 ms; curved N=4 K=1296 (6
+// steps) 12.4 -> 10.4, curved N=3 K=3072 9.0 -> 7.3, 7986 tets N=2 5.9 -> 4.8, 2D
+// N=3 K=8192 3.33 -> 3.18; errors against autodiff in 64 bits as before (4e-16).
+template <int DIM> struct PairNode {
+  double hr, h[DIM], beta, lrho, lbeta;
+};
+
+template <int DIM, int TT>
+__device__ __forceinline__ void pair_vjp(const PairNode<DIM> &a, const PairNode<DIM> &b, const double *n,
+                                         const double *c, const Phys &P, double *ba, double *bb) {
+  constexpr int TP = TT < 2 ? TT : 2;
+  const double sr = a.hr + b.hr, dr = a.hr - b.hr, db = a.beta - b.beta;
+  const double isb = rcp(a.beta + b.beta);
+  const double fr = dr * (TT == 0 ? rcp1(sr) : rcp(sr)), fb = db * isb;
+  const double ur = fr * fr, ub = fb * fb;
+  const double pa = sr * isb;
+  double rl, rla, rlb, ib, ka, iba, ibb;  // the means; d rl; d ib = ka (iba, ibb)
+  const double m = P.igm1 * isb;
+  auto series_r = [&] {
+    const double G = polyG<TP>(ur), T = poly2dG<TP>(ur) * fr, w = fma(-T, fr, G);
+    rl = sr * G;
+    rla = w + T;
+    rlb = w - T;
+  };
+  auto series_b = [&] {
+    const double F = polyF<TP>(ub), S = poly2dF<TP>(ub) * fb, w = fma(-S, fb, -F);
+    ib = m * F;
+    ka = m * isb;
+    iba = w + S;
+    ibb = w - S;
+  };
+  if (TT < 3) {
+    series_r();
+    series_b();
+  } else {
+    if (ur < logmean_u(2)) {
+      series_r();
+    } else {
+      const double ild = rcp(a.lrho - b.lrho);
+      rl = 2.0 * dr * ild;
+      rla = 2.0 * ild * fma(-0.5 * rl, rcp(a.hr), 1.0);
+      rlb = 2.0 * ild * fma(0.5 * rl, rcp(b.hr), -1.0);
+    }
+    if (ub < logmean_u(2)) {
+      series_b();
+    } else {
+      ka = rcp(db);
+      ib = P.cbeta * (a.lbeta - b.lbeta) * ka;
+      iba = fma(P.cbeta, rcp(a.beta), -ib);
+      ibb = fma(-P.cbeta, rcp(b.beta), ib);
+    }
+  }
+  double ubar[DIM], un = 0.0, cu = c[0], cn = 0.0, q = 0.0;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) {
+    ubar[d] = a.h[d] + b.h[d];
+    un = d ? fma(ubar[d], n[d], un) : ubar[d] * n[d];
+    cu = fma(c[1 + d], ubar[d], cu);
+    cn = d ? fma(c[1 + d], n[d], cn) : c[1 + d] * n[d];
+    q = d ? fma(a.h[d], b.h[d], q) : a.h[d] * b.h[d];
+  }
+  const double cE = c[DIM + 1];
+  const double hh = fma(2.0, q, ib), f4 = fma(rl, hh, pa), F0 = rl * un;
+  const double f4b = cE * un;
+  const double unb = fma(cu, rl, cE * f4);
+  const double rlbar = fma(cu, un, f4b * hh);
+  const double g = f4b * rl, g2 = 2.0 * g, gk = g * ka;
+  const double pr = (cn + f4b) * isb, pb = -pr * pa;
+  ba[0] = fma(rlbar, rla, ba[0] + pr);
+  bb[0] = fma(rlbar, rlb, bb[0] + pr);
+  ba[DIM + 1] = fma(gk, iba, ba[DIM + 1] + pb);
+  bb[DIM + 1] = fma(gk, ibb, bb[DIM + 1] + pb);
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) {
+    const double hb = fma(c[1 + d], F0, unb * n[d]);
+    ba[1 + d] = fma(g2, b.h[d], ba[1 + d] + hb);
+    bb[1 + d] = fma(g2, a.h[d], bb[1 + d] + hb);
+  }
+}
+
+// Surface term (once per face point, two seeds per state pair): the part that depends on
+// the two states only (FluxCore: the means and their partial derivatives, in rho, u
+// and beta) and a reverse sweep per (n, c) that adds a's adjoint.
 template <int DIM> struct FluxCore {
-  double rl, rla, rlb, ibl, ibla, iblb, pa, isb, ubar[DIM], vv;
+  double rl, rla, ibl, ibla, pa, isb, ubar[DIM], vv;
 };
 
-__device__ __forceinline__ void rl_series(double sr, double fr, double G, double dG, double &rl,
-                                          double &rla, double &rlb) {
-  rl = 0.5 * sr * G;
-  const double t = dG * fr;
-  rla = fma(-t, fr, fma(0.5, G, t));
-  rlb = fma(-t, fr, fma(0.5, G, -t));
-}
-__device__ __forceinline__ void ibl_series(double isb, double fb, double F, double dF,
-                                           double &ibl, double &ibla, double &iblb) {
-  ibl = 2.0 * isb * F;
-  const double t2 = 2.0 * isb * isb, t = 2.0 * dF * fb;
-  ibla = t2 * (fma(-t, fb, t) - F);
-  iblb = t2 * (fma(-t, fb, -t) - F);
-}
-
-template <bool B> struct BoolTag {
-  static constexpr bool value = B;
-};
-constexpr double SMALL_U = 4e-6;
-
-// WARP = true: must be called by all 32 lanes of a converged warp; when every
-// lane has u < 1e-6 for both means (nearly equal states, e.g. the whole
-// Taylor-Green field) the series are truncated at u^2 (remainders below
-// 1e-18 relative in the means and 1e-13 in their u-derivatives, which enter
-// multiplied by f < 1e-3).  SMALL = true: the caller has established u <
-// SMALL_U (4e-6) for every pair of the warp's elements (state_spread); the
-// truncated series without a vote (remainders below 1e-17 in the means and
-// 2e-11 in the derivatives, which enter multiplied by f < 2e-3).
-template <int DIM, bool WARP, bool SMALL = false>
+template <int DIM>
 __device__ __forceinline__ FluxCore<DIM> flux_core(const AdjNode<DIM> &a, const AdjNode<DIM> &b) {
   FluxCore<DIM> k;
   const double sr = a.rho + b.rho, dr = a.rho - b.rho;
   const double sb = a.beta + b.beta, db = a.beta - b.beta;
-  const double isr = rcp1(sr);  // forms only the series argument and f(1 -+ f)
   k.isb = rcp(sb);
-  const double fr = dr * isr, fb = db * k.isb;
+  const double fr = dr * rcp(sr), fb = db * k.isb;
   const double ur = fr * fr, ub = fb * fb;
-  if (SMALL || (WARP && __all_sync(0xffffffffu, fmax(ur, ub) < 1e-6))) {
-    rl_series(sr, fr, fma(fma(ur, -4.0 / 45.0, -1.0 / 3.0), ur, 1.0), fma(ur, -8.0 / 45.0, -1.0 / 3.0),
-              k.rl, k.rla, k.rlb);
-    ibl_series(k.isb, fb, fma(fma(ub, 1.0 / 5.0, 1.0 / 3.0), ub, 1.0), fma(ub, 2.0 / 5.0, 1.0 / 3.0),
-               k.ibl, k.ibla, k.iblb);
-  } else if (WARP && __all_sync(0xffffffffu, fmax(ur, ub) < 1e-2)) {
-    // every lane in the degree-8 series range for both means: the same
-    // series as below, with no per-lane branch
-    double G, dG, F, dF;
-    polyG_d(ur, G, dG);
-    rl_series(sr, fr, G, dG, k.rl, k.rla, k.rlb);
-    polyF_d(ub, F, dF);
-    ibl_series(k.isb, fb, F, dF, k.ibl, k.ibla, k.iblb);
+  if (ur < logmean_u(2)) {
+    const double G = polyG<2>(ur), t = 0.5 * poly2dG<2>(ur) * fr;
+    k.rl = 0.5 * sr * G;
+    k.rla = fma(-t, fr, fma(0.5, G, t));
   } else {
-    if (ur < 1e-2) {
-      double G, dG;
-      polyG_d(ur, G, dG);
-      rl_series(sr, fr, G, dG, k.rl, k.rla, k.rlb);
-    } else {
-      const double ild = rcp(a.lrho - b.lrho);
-      k.rl = dr * ild;
-      k.rla = fma(-k.rl, a.irho, 1.0) * ild;
-      k.rlb = fma(k.rl, b.irho, -1.0) * ild;
-    }
-    if (ub < 1e-2) {
-      double F, dF;
-      polyF_d(ub, F, dF);
-      ibl_series(k.isb, fb, F, dF, k.ibl, k.ibla, k.iblb);
-    } else {
-      const double idb = rcp(db);
-      k.ibl = (a.lbeta - b.lbeta) * idb;
-      k.ibla = (a.ibeta - k.ibl) * idb;
-      k.iblb = (k.ibl - b.ibeta) * idb;
-    }
+    const double ild = rcp(log(a.rho * b.irho));
+    k.rl = dr * ild;
+    k.rla = fma(-k.rl, a.irho, 1.0) * ild;
+  }
+  if (ub < logmean_u(2)) {
+    const double F = polyF<2>(ub), t = poly2dF<2>(ub) * fb;
+    k.ibl = 2.0 * k.isb * F;
+    k.ibla = 2.0 * k.isb * k.isb * (fma(-t, fb, t) - F);
+  } else {
+    const double idb = rcp(db);
+    k.ibl = log(a.beta * b.ibeta) * idb;
+    k.ibla = (a.ibeta - k.ibl) * idb;
   }
   k.pa = 0.5 * sr * k.isb;
   k.vv = 0.0;
@@ -168,11 +231,10 @@ __device__ __forceinline__ FluxCore<DIM> flux_core(const AdjNode<DIM> &a, const 
   return k;
 }
 
-// reverse sweep for one direction n and adjoint c; BSIDE = false skips b's adjoint
-template <int DIM, bool BSIDE>
-__device__ __forceinline__ void flux_rev(const FluxCore<DIM> &k, const AdjNode<DIM> &a,
-                                         const AdjNode<DIM> &b, const double *n, const double *c,
-                                         const Phys &P, double *ba, double *bb) {
+// reverse sweep for one direction n and adjoint c: a's adjoint
+template <int DIM>
+__device__ __forceinline__ void flux_rev(const FluxCore<DIM> &k, const AdjNode<DIM> &b, const double *n,
+                                         const double *c, const Phys &P, double *ba) {
   double un = 0.0, cu = 0.0, cn = 0.0;
 #pragma unroll
   for (int d = 0; d < DIM; ++d) {
@@ -194,24 +256,11 @@ __device__ __forceinline__ void flux_rev(const FluxCore<DIM> &k, const AdjNode<D
   const double prho = 0.5 * pab * k.isb, pbeta = -pab * k.pa * k.isb;
   ba[0] = fma(rlbar, k.rla, ba[0] + prho);
   ba[DIM + 1] = fma(iblbar, k.ibla, ba[DIM + 1] + pbeta);
-  if (BSIDE) {
-    bb[0] = fma(rlbar, k.rlb, bb[0] + prho);
-    bb[DIM + 1] = fma(iblbar, k.iblb, bb[DIM + 1] + pbeta);
-  }
 #pragma unroll
   for (int d = 0; d < DIM; ++d) {
     const double hb = 0.5 * fma(c[1 + d], F0, unb * n[d]);
     ba[1 + d] = fma(vvb, b.vel[d], ba[1 + d] + hb);
-    if (BSIDE) bb[1 + d] = fma(vvb, a.vel[d], bb[1 + d] + hb);
   }
-}
-
-template <int DIM, bool WARP, bool SMALL = false>
-__device__ __forceinline__ void ecflux_vjp(const AdjNode<DIM> &a, const AdjNode<DIM> &b,
-                                           const double *n, const double *c, const Phys &P,
-                                           double *ba, double *bb) {
-  const FluxCore<DIM> k = flux_core<DIM, WARP, SMALL>(a, b);
-  flux_rev<DIM, true>(k, a, b, n, c, P, ba, bb);
 }
 
 // adjoint of the primitive recovery (rho, u = m/rho, beta = rho/(2p)) at a
@@ -262,8 +311,6 @@ __device__ __forceinline__ AdjNode<DIM> adj_node(const double *q, const Phys &P)
 #pragma unroll
   for (int d = 0; d < DIM; ++d) a.vel[d] = s.vel[d];
   a.beta = s.beta;
-  a.lrho = log(s.rho);
-  a.lbeta = log(s.beta);
   a.irho = rcp(s.rho);
   a.ibeta = rcp(s.beta);
   return a;
@@ -294,7 +341,7 @@ struct AdjPairsCfg {
   static constexpr int L = T::L, R = T::R, G = T::G;
   static constexpr int nv0 = (Nq + 1) / 2, nv1 = Nq - nv0, nf0 = (NF + 1) / 2, nf1 = NF - nf0;
   static constexpr int H = (nv1 >= L && nf1 >= L) ? 2 : 1;
-  static constexpr int NSA = DIM + 6;               // AdjNode fields
+  static constexpr int NSA = DIM + 4;               // rho/2, u/2, beta, log rho, log beta
   static constexpr int NGS = CURVED ? El::Nvgeo : 0; // geometric factors per node
   static constexpr int NB = DIM + 2;                // primitive adjoint components
   static constexpr int threads = 32 * W;
@@ -453,21 +500,17 @@ adj_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
           if (c0 + j < NT && t < G * NN) {
             const int ee = e0 + t / NN, n = t % NN;
             const int k = min(k0 + ee, K - 1);
-            const AdjNode<DIM> s = adj_node<DIM>(u[j], P);
+            const NodeState<DIM> s = node_state<DIM>(u[j], P);
             double *st = sEl + ee * C::per_elem;
-            st[0 * NN + n] = s.rho;
+            st[0 * NN + n] = 0.5 * s.rho;
 #pragma unroll
-            for (int d = 0; d < DIM; ++d) st[(1 + d) * NN + n] = s.vel[d];
+            for (int d = 0; d < DIM; ++d) st[(1 + d) * NN + n] = 0.5 * s.vel[d];
             st[(DIM + 1) * NN + n] = s.beta;
-            st[(DIM + 2) * NN + n] = s.lrho;
-            st[(DIM + 3) * NN + n] = s.lbeta;
-            st[(DIM + 4) * NN + n] = s.irho;
-            st[(DIM + 5) * NN + n] = s.ibeta;
-            if (CURVED) {
+            if (CURVED) {  // halved: a pair's average is a sum
 #pragma unroll
               for (int c = 0; c < NG; ++c)
-                st[(NSA + c) * NN + n] = (n < Nq) ? vgeo[(size_t)k * Nq * NG + c * Nq + n]
-                                                  : vfgeo[(size_t)k * NF * NG + c * NF + (n - Nq)];
+                st[(NSA + c) * NN + n] = 0.5 * ((n < Nq) ? vgeo[(size_t)k * Nq * NG + c * Nq + n]
+                                                         : vfgeo[(size_t)k * NF * NG + c * NF + (n - Nq)]);
             }
           }
         }
@@ -509,27 +552,27 @@ adj_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
     const double *sfb = st + C::SST;
     double *bar = sEl + e * C::per_elem + C::SST + C::SSF;
     const double *nm = st + C::SST + C::SSF + C::SBR;
-    auto load = [&](int n) {
-      AdjNode<DIM> s;
-      s.rho = st[n];
+    auto load = [&](auto range, int n) {
+      PairNode<DIM> s;
+      s.hr = st[n];
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) s.vel[d] = st[(1 + d) * NN + n];
+      for (int d = 0; d < DIM; ++d) s.h[d] = st[(1 + d) * NN + n];
       s.beta = st[(DIM + 1) * NN + n];
-      s.lrho = st[(DIM + 2) * NN + n];
-      s.lbeta = st[(DIM + 3) * NN + n];
-      s.irho = st[(DIM + 4) * NN + n];
-      s.ibeta = st[(DIM + 5) * NN + n];
+      s.lrho = s.lbeta = 0.0;
+      if (decltype(range)::value == 3) {
+        s.lrho = st[(DIM + 2) * NN + n];
+        s.lbeta = st[(DIM + 3) * NN + n];
+      }
       return s;
     };
     const int kq = min(k0 + e, K - 1);
-    AdjNode<DIM> A[R];
+    PairNode<DIM> A[R];
     int ir[R];
     double cr[R][Nf], rb[R][NB];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int i = l + L * r;
       ir[r] = min(i, Nq - 1);  // padding row: clamped state, zero seed
-      A[r] = load(ir[r]);
 #pragma unroll
       for (int q = 0; q < Nf; ++q)
         cr[r][q] = i < Nq ? rhsbar[(size_t)kq * Nq * Nf + q * Nq + i] : 0.0;
@@ -542,10 +585,11 @@ adj_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
       for (int c = 0; c < NG; ++c) Ge[c] = nm[El::Nfaces * DIM + c];
     }
 
-    // the pair loops: with a vote per pair (SM = false) or, where every pair
-    // of the warp's elements is nearly equal (state_spread), without
-    auto pair_loops = [&](auto small_tag) {
-    constexpr bool SM = decltype(small_tag)::value;
+    // the pair loops for one range of the states (state_range)
+    auto pair_loops = [&](auto range) {
+    constexpr int TT = decltype(range)::value;
+#pragma unroll
+    for (int r = 0; r < R; ++r) A[r] = load(range, ir[r]);
     // volume-volume pairs over this warp's column half
     {
       const int n_ = nv(h), j0 = cv(h);
@@ -553,7 +597,7 @@ adj_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
         int jj = l + s;
         if (jj >= n_) jj -= n_;
         const int j = j0 + jj;
-        const AdjNode<DIM> B = load(j);
+        const PairNode<DIM> B = load(range, j);
         double cb[NB];
 #pragma unroll
         for (int q = 0; q < NB; ++q) cb[q] = 0.0;
@@ -567,14 +611,14 @@ adj_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
             double v = 0.0;
 #pragma unroll
             for (int a = 0; a < DIM; ++a) {
-              const double gad = CURVED ? 0.5 * (st[(NSA + a * DIM + d) * NN + ir[r]] +
-                                                 st[(NSA + a * DIM + d) * NN + j])
+              const double gad = CURVED ? st[(NSA + a * DIM + d) * NN + ir[r]] +
+                                              st[(NSA + a * DIM + d) * NN + j]
                                         : Ge[a * DIM + d];
               v = fma(gad, rr[a], v);
             }
             nvd[d] = v;
           }
-          ecflux_vjp<DIM, !SM, SM>(A[r], B, nvd, cr[r], P, rb[r], cb);
+          pair_vjp<DIM, TT>(A[r], B, nvd, cr[r], P, rb[r], cb);
         }
 #pragma unroll
         for (int q = 0; q < NB; ++q) bar[q * NN + j] += cb[q];
@@ -588,7 +632,7 @@ adj_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
         int ff = l + s;
         if (ff >= n_) ff -= n_;
         const int f = f0 + ff;
-        const AdjNode<DIM> B = load(Nq + f);
+        const PairNode<DIM> B = load(range, Nq + f);
         const int fc = f / Nfq;
         double cfs[Nf], nvd[DIM];
 #pragma unroll
@@ -608,8 +652,7 @@ adj_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
               double v = 0.0;
 #pragma unroll
               for (int a = 0; a < DIM; ++a)
-                v = fma(0.5 * (st[(NSA + a * DIM + d) * NN + ir[r]] +
-                               st[(NSA + a * DIM + d) * NN + Nq + f]),
+                v = fma(st[(NSA + a * DIM + d) * NN + ir[r]] + st[(NSA + a * DIM + d) * NN + Nq + f],
                         sNr[fc * DIM + a], v);
               nvd[d] = v;
             }
@@ -619,7 +662,7 @@ adj_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
           double c[Nf];
 #pragma unroll
           for (int q = 0; q < Nf; ++q) c[q] = fma(w1, cr[r][q], w2 * cfs[q]);
-          ecflux_vjp<DIM, !SM, SM>(A[r], B, nvd, c, P, rb[r], cb);
+          pair_vjp<DIM, TT>(A[r], B, nvd, c, P, rb[r], cb);
         }
 #pragma unroll
         for (int q = 0; q < NB; ++q) bar[q * NN + Nq + f] += cb[q];
@@ -627,14 +670,25 @@ adj_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
       }
     }
     };
-    const double spread = state_spread<NN, L>(l, [&](int n, int &r, int &b) {
+    const int range = state_range<NN, L>(l, [&](int n, int &r, int &b) {
       r = __double2hiint(st[n]);
       b = __double2hiint(st[(DIM + 1) * NN + n]);
     });
-    if (__all_sync(0xffffffffu, spread < SMALL_U))
-      pair_loops(BoolTag<true>());
-    else
-      pair_loops(BoolTag<false>());
+    if (range == 0) {
+      pair_loops(IntTag<0>());
+    } else if (range == 1) {
+      pair_loops(IntTag<1>());
+    } else if (range == 2) {
+      pair_loops(IntTag<2>());
+    } else {
+      for (int t = tq; t < G * NN; t += GT) {  // the logarithms, only here
+        double *sl = sEl + (e0 + t / NN) * C::per_elem + t % NN;
+        sl[(DIM + 2) * NN] = log(2.0 * sl[0]);
+        sl[(DIM + 3) * NN] = log(sl[(DIM + 1) * NN]);
+      }
+      gsync();
+      pair_loops(IntTag<3>());
+    }
     // row adjoints into the column adjoints, one warp of the element at a time
 #pragma unroll
     for (int hh = 0; hh < H; ++hh) {
@@ -659,17 +713,16 @@ adj_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
       const double *ste = sEl + ee * C::per_elem;
       const double *bt = ste + C::SST + C::SSF;
       AdjNode<DIM> own;
-      own.rho = ste[n];
+      own.rho = 2.0 * ste[n];
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) own.vel[d] = ste[(1 + d) * NN + n];
+      for (int d = 0; d < DIM; ++d) own.vel[d] = 2.0 * ste[(1 + d) * NN + n];
       own.beta = ste[(DIM + 1) * NN + n];
-      own.lrho = ste[(DIM + 2) * NN + n];
-      own.lbeta = ste[(DIM + 3) * NN + n];
-      own.irho = ste[(DIM + 4) * NN + n];
-      own.ibeta = ste[(DIM + 5) * NN + n];
+      own.irho = rcp(own.rho);
+      own.ibeta = rcp(own.beta);
+      // the pair phase's adjoints are those of rho/2 and u/2
       double pb[NB], U[Nf], Ub[Nf], Vb[Nf];
 #pragma unroll
-      for (int q = 0; q < NB; ++q) pb[q] = bt[q * NN + n];
+      for (int q = 0; q < NB; ++q) pb[q] = (q <= DIM ? 0.5 : 1.0) * bt[q * NN + n];
       if (n < Nq) {
         const double *qv = uq + (size_t)k * Nq * Nf + n;
 #pragma unroll
@@ -704,9 +757,9 @@ adj_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
         }
         const double sJM = fgM[DIM * NF], sJP = fgP[DIM * NF];
         const AdjNode<DIM> nb = adj_node<DIM>(UP, P);
-        const FluxCore<DIM> core = flux_core<DIM, false>(own, nb);
-        flux_rev<DIM, false>(core, own, nb, nM, cM, P, pb, nullptr);
-        flux_rev<DIM, false>(core, own, nb, nP, cP, P, pb, nullptr);
+        const FluxCore<DIM> core = flux_core<DIM>(own, nb);
+        flux_rev<DIM>(core, nb, nM, cM, P, pb);
+        flux_rev<DIM>(core, nb, nP, cP, P, pb);
         prim_vjp_dev<DIM>(own, pb, P, Ub);
         double dl[Nf];
         const double lamM = lambda_dev<DIM, true>(own, P, dl);
