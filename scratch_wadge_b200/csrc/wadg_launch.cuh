@@ -179,6 +179,23 @@ bool small_mesh(const wadg_ctx *c, int K) {
   return per_sm <= groups;
 }
 
+// Warps per CTA of the default map: the context's choice, else the default (0), or 16
+// in 2D where they finish in a round fewer (at most two, as their 128
+// registers per thread cost 2 % in longer runs).  10 time steps, ms, 12 -> 16
+// warps, by slices per SM: N=3 (6 groups for 8) 6.9 1.318 -> 1.223, 13.8 2.10 ->
+// 2.02; curved N=3 6.9 1.58 -> 1.44; N=2 13.8 2.31 -> 2.17; curved N=2 6.9 1.70 ->
+// 1.53; curved N=4 (12 groups for 16) 12.2 2.05 -> 1.83, affine N=4 13.8 (not
+// taken) 1.79 -> 1.81.  Same bits
+template <int DIM, int N, bool CURVED>
+int default_warps(const wadg_ctx *c, int K) {
+  constexpr int W0 = volpairsW<DIM, N, CURVED>(), W1 = volpairsW_cand<DIM, N, CURVED>(1);
+  if (c->vol_warps || c->vol_rows || DIM == 3 || (N == 4 && !CURVED) || W1 <= W0) return c->vol_warps;
+  constexpr int g0 = W0 / VolTile<DIM, N>::H, g1 = W1 / VolTile<DIM, N>::H;
+  const int slices = (K + VolTile<DIM, N>::G - 1) / VolTile<DIM, N>::G;
+  const int m = (slices + num_sms() - 1) / num_sms();
+  return m <= 2 * g1 && (m + g1 - 1) / g1 < (m + g0 - 1) / g0 ? W1 : 0;
+}
+
 // SURF: the volume + surface kernel (rhsQf unused; fgeo, mapPq read)
 template <int DIM, int N, bool CURVED, int W, bool SURF = false, int RR = 0, int HH = 0>
 int launch_vol_pairs_w(const wadg_ctx *c, int K, const double *vgeo, const double *vfgeo,
@@ -228,11 +245,12 @@ int launch_volsurf(const wadg_ctx *c, int K, const double *vgeo, const double *v
           c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, nullptr, fgeo,
           mapPq, blist, nb);
   constexpr int W1 = volpairsW_cand<DIM, N, CURVED>(1), W2 = volpairsW_cand<DIM, N, CURVED>(2);
-  if (W1 && c->vol_warps == W1)
+  const int warps = default_warps<DIM, N, CURVED>(c, K);
+  if (W1 && warps == W1)
     return launch_vol_pairs_w<DIM, N, CURVED, (W1 ? W1 : 2), true>(
         c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, nullptr, fgeo, mapPq,
         blist, nb);
-  if (W2 && c->vol_warps == W2)
+  if (W2 && warps == W2)
     return launch_vol_pairs_w<DIM, N, CURVED, (W2 ? W2 : 2), true>(
         c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, nullptr, fgeo, mapPq,
         blist, nb);
@@ -262,10 +280,11 @@ int launch_vol_pairs(const wadg_ctx *c, int K, const double *vgeo, const double 
       return launch_vol_pairs_w<DIM, N, CURVED, alt_warps<DIM, N, CURVED, A1>(), false, A1>(
           c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, rhsQf);
   constexpr int W1 = volpairsW_cand<DIM, N, CURVED>(1), W2 = volpairsW_cand<DIM, N, CURVED>(2);
-  if (W1 && c->vol_warps == W1)
+  const int warps = default_warps<DIM, N, CURVED>(c, K);
+  if (W1 && warps == W1)
     return launch_vol_pairs_w<DIM, N, CURVED, (W1 ? W1 : 2)>(c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq,
                                                              Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, rhsQf);
-  if (W2 && c->vol_warps == W2)
+  if (W2 && warps == W2)
     return launch_vol_pairs_w<DIM, N, CURVED, (W2 ? W2 : 2)>(c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq,
                                                              Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, rhsQf);
   return launch_vol_pairs_w<DIM, N, CURVED, volpairsW<DIM, N, CURVED>()>(
@@ -378,10 +397,11 @@ int kernel_shape(const wadg_ctx *c, int kernel, int K, int *E, int *grid) {
       vol_shape<DIM, N, CURVED, 12, 0, HH>(K, E, grid);
       return WADG_OK;
     }
+  const int warps = default_warps<DIM, N, CURVED>(c, K);
   switch (kernel) {
     case WADG_KERNEL_VOL:
-      if (W1 && c->vol_warps == W1) vol_shape<DIM, N, CURVED, (W1 ? W1 : 2)>(K, E, grid);
-      else if (W2 && c->vol_warps == W2) vol_shape<DIM, N, CURVED, (W2 ? W2 : 2)>(K, E, grid);
+      if (W1 && warps == W1) vol_shape<DIM, N, CURVED, (W1 ? W1 : 2)>(K, E, grid);
+      else if (W2 && warps == W2) vol_shape<DIM, N, CURVED, (W2 ? W2 : 2)>(K, E, grid);
       else vol_shape<DIM, N, CURVED, volpairsW<DIM, N, CURVED>()>(K, E, grid);
       return WADG_OK;
     case WADG_KERNEL_SURF:
@@ -392,8 +412,8 @@ int kernel_shape(const wadg_ctx *c, int kernel, int K, int *E, int *grid) {
       *E = UpdMmaCfg<DIM, N, CURVED>::EW;
       return update_grid<DIM, N, CURVED>(K, grid);
     case WADG_KERNEL_VOLSURF:  // the same CTA shapes as the volume kernel
-      if (W1 && c->vol_warps == W1) vol_shape<DIM, N, CURVED, (W1 ? W1 : 2)>(K, E, grid);
-      else if (W2 && c->vol_warps == W2) vol_shape<DIM, N, CURVED, (W2 ? W2 : 2)>(K, E, grid);
+      if (W1 && warps == W1) vol_shape<DIM, N, CURVED, (W1 ? W1 : 2)>(K, E, grid);
+      else if (W2 && warps == W2) vol_shape<DIM, N, CURVED, (W2 ? W2 : 2)>(K, E, grid);
       else vol_shape<DIM, N, CURVED, volpairsW<DIM, N, CURVED>()>(K, E, grid);
       return WADG_OK;
     case WADG_KERNEL_ADJ_PAIRS:
