@@ -54,7 +54,10 @@ __device__ __forceinline__ void prefetch_lines(const void *p, int bytes, int t0,
 
 // Programmatic dependent launch: let the next kernel of the stream start its
 // preamble, and wait for the previous one to finish (both do nothing in a
-// kernel launched without the attribute)
+// kernel launched without the attribute).  What a predecessor writes may change
+// while such a kernel already runs, so its pointers are neither const __restrict__
+// nor read by __ldg: both promise data that is constant for the whole kernel,
+// which lets a load take the non-coherent path or move above the wait
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 

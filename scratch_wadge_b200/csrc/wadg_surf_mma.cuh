@@ -40,8 +40,8 @@ struct SurfMmaCfg {
 template <int DIM, int N>
 __global__ void __launch_bounds__(SurfMmaCfg<DIM, N>::threads, SurfMmaCfg<DIM, N>::min_ctas)
 surf_mma_kernel(int K, const double *__restrict__ fgeo, const uint32_t *__restrict__ mapPq,
-                const double *__restrict__ VqLq, const double *__restrict__ Qf,
-                const double *__restrict__ rhsQf, double *__restrict__ rhsQ, Phys P) {
+                const double *__restrict__ VqLq, const double *Qf, const double *rhsQf,
+                double *rhsQ, Phys P) {
   using C = SurfMmaCfg<DIM, N>;
   using El = Elem<DIM, N>;
   constexpr int Nq = C::Nq, NF = C::NF, Nf = C::Nf, EW = C::EW, KSF = C::KSF, KPF = C::KPF,

@@ -323,7 +323,7 @@ __device__ __forceinline__ void stage_rhs(const double *rhs, int k0, int ne, dou
 #pragma unroll
   for (int it = 0; it < IT; ++it) {
     const int t = tid + THREADS * it;
-    v[it] = t < lim ? (CG ? __ldcg(src + t) : __ldg(src + t)) : 0.0;
+    v[it] = t < lim ? (CG ? __ldcg(src + t) : src[t]) : 0.0;
   }
   between();
   sync();  // the previous group's last reads of X and Y are done
@@ -342,8 +342,8 @@ template <int DIM, int N, bool CURVED, bool WIDE = false>
 __global__ void __launch_bounds__(UpdMmaCfg<DIM, N, CURVED, WIDE>::threads, UpdMmaCfg<DIM, N, CURVED, WIDE>::min_ctas)
 update_mma_kernel(int K, const double *__restrict__ Jq, const double *__restrict__ VqPq,
                   const double *__restrict__ VfPq, double fa, double fb, double fdt,
-                  double *__restrict__ rhsQ, double *__restrict__ resQ, double *__restrict__ Q,
-                  double *__restrict__ Qf, Phys P, const double *__restrict__ dtK = nullptr,
+                  double *rhsQ, double *resQ, double *Q, double *Qf, Phys P,
+                  const double *__restrict__ dtK = nullptr,
                   const int *__restrict__ blist = nullptr, const int *__restrict__ nblist = nullptr) {
   using C = UpdMmaCfg<DIM, N, CURVED, WIDE>;
   constexpr int Nq = C::Nq, Nf = C::Nf, EW = C::EW, KP = C::KP, LD = C::LD, MQ = C::MQ;

@@ -691,8 +691,8 @@ struct VolPairs {
   template <int TS>
   __device__ __forceinline__ void surface(int K, int k0, int e0, int t0,
                                           const double *__restrict__ fgeo,
-                                          const uint32_t *__restrict__ mapPq,
-                                          const double *__restrict__ uf, const Phys &P) const {
+                                          const uint32_t *__restrict__ mapPq, const double *uf,
+                                          const Phys &P) const {
     constexpr int NFG = El::Nfgeo, NPT = (G * NF + TS - 1) / TS;
     // point u of the thread: its element (in the group) and face node; those
     // past the group's or the mesh's end repeat a valid one and are not stored
@@ -844,8 +844,8 @@ vol_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
                  const double *__restrict__ ntJ, const double *__restrict__ Drq,
                  const double *__restrict__ Dsq, const double *__restrict__ Dtq,
                  const double *__restrict__ VqLq, const double *__restrict__ VfPq,
-                 const double *__restrict__ Qf, double *__restrict__ rhsQ,
-                 double *__restrict__ rhsQf, Phys P, const double *__restrict__ fgeo = nullptr,
+                 const double *Qf, double *rhsQ, double *rhsQf, Phys P,
+                 const double *__restrict__ fgeo = nullptr,
                  const uint32_t *__restrict__ mapPq = nullptr,
                  const int *__restrict__ blist = nullptr, const int *__restrict__ nblist = nullptr) {
   using V = VolPairs<DIM, N, CURVED, W, RR, HH>;
