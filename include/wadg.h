@@ -454,11 +454,13 @@ int wadg_app_time_volsurf(wadg_app *app, double dt, int nstages, float *ms);
  * CTA shape of the volume kernel -- or, in the volume + surface stage
  * variant, of the volume + surface kernel, which has the same shapes -- on
  * the app's own mesh and state, over every shape of wadg_vol_shapes (CTA
- * size and node-to-thread map), keeps the fastest (its warps written to
- * *warps, its rows to be read with wadg_ctx_get_vol_rows; times, if not NULL,
- * an array of WADG_MAX_VOL_SHAPES, receives that kernel's ms per launch for
- * each shape in the order of wadg_vol_shapes) and leaves it selected for the
- * app's kernels.  Advances the app's state: call it before set_state. */
+ * size and node-to-thread map) and, on a small mesh, the automatic shape,
+ * which is none of those; keeps the fastest (its warps written to *warps, 0
+ * for the automatic shape, its rows to be read with wadg_ctx_get_vol_rows;
+ * times, if not NULL, an array of WADG_MAX_VOL_SHAPES, receives that kernel's
+ * ms per launch for each shape in the order of wadg_vol_shapes -- for the
+ * first, the better of its own and the automatic shape's) and leaves it
+ * selected for the app's kernels.  Advances the app's state: call it before set_state. */
 int wadg_app_autotune(wadg_app *app, double dt, int nstages, int *warps,
                       float *times);
 

@@ -437,13 +437,17 @@ class App:
         map) by timing each compiled one on this app (advances the state: set
         it afterwards).  Returns (the chosen shape, {shape: ms per launch});
         a shape is its warps per CTA ("12") or, for another map than the
-        default, warps and rows per lane ("16w2r")."""
+        default, warps and rows per lane ("16w2r").  On a small mesh the
+        automatic shape is timed beside the first; where it wins, it stands
+        in the first's place as "0"."""
         w = ctypes.c_int()
         t = (ctypes.c_float * MAX_VOL_SHAPES)()
         check(lib().wadg_app_autotune(self.h, dt, nstages, ctypes.byref(w), t), "autotune")
         ctx = ctypes.c_void_p(lib().wadg_app_ctx(self.h))
         shapes = vol_shapes(ctx, self.curved)
         rows = lib().wadg_ctx_get_vol_rows(ctx)
+        if w.value == 0:
+            shapes[0] = (0, 0)
         return shape_label(w.value, rows), {shape_label(a, b): float(t[k]) for k, (a, b) in enumerate(shapes)}
 
     def vol_shape(self):

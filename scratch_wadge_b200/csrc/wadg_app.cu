@@ -9,6 +9,7 @@
 
 #include "../../include/wadg.h"
 #include "wadg_app_impl.h"
+#include "wadg_host.h"
 
 namespace wadg_internal {
 void set_error(const std::string &msg);  // wadg_capi.cu
@@ -494,18 +495,24 @@ int wadg_app_autotune(wadg_app *a, double dt, int nstages, int *warps, float *ti
   int cw[WADG_MAX_VOL_SHAPES], cr[WADG_MAX_VOL_SHAPES];
   const int n = wadg_vol_shapes(a->ctx, a->curved, cw, cr);
   if (n <= 0) return afail(WADG_ERR_UNSUPPORTED, "no volume kernel shapes");
+  // on a small mesh the automatic shape (0) is none of the listed ones: timed
+  // beside the first, which is the default's number elsewhere
+  const int nt = n + (wadg_internal::vol_automatic(a->ctx, a->curved, a->K) ? 1 : 0);
   int best = 0;
   float best_ms = -1.0f;
   // the volume kernel's time, or (volume + surface variant) the volume +
   // surface kernel's
   const bool vs = a->fused == WADG_STAGE_VOLSURF;
-  for (int i = 0; i < n; ++i) {
-    int r = wadg_ctx_set_vol_shape(a->ctx, a->curved, cw[i], cr[i]);
+  for (int i = 0; i < nt; ++i) {
+    const int w = i < n ? cw[i] : 0, rows = i < n ? cr[i] : 0;
+    int r = wadg_ctx_set_vol_shape(a->ctx, a->curved, w, rows);
     float ms[3] = {0, 0, 0};
     if (!r) r = vs ? wadg_app_time_volsurf(a, dt, 1, ms) : wadg_app_time_kernels(a, dt, 1, ms);
     if (!r) r = vs ? wadg_app_time_volsurf(a, dt, nstages, ms) : wadg_app_time_kernels(a, dt, nstages, ms);
     if (r) return r;
-    if (times) times[i] = ms[0] / nstages;
+    const float t = ms[0] / nstages;
+    if (times && i < n) times[i] = t;
+    if (times && i == n && t < times[0]) times[0] = t;
     if (best_ms < 0.0f || ms[0] < best_ms) {
       best_ms = ms[0];
       best = i;
@@ -517,8 +524,9 @@ int wadg_app_autotune(wadg_app *a, double dt, int nstages, int *warps, float *ti
       cudaGraphExecDestroy(g);
       g = nullptr;
     }
-  if (warps) *warps = cw[best];
-  return wadg_ctx_set_vol_shape(a->ctx, a->curved, cw[best], cr[best]);
+  const int w = best < n ? cw[best] : 0;
+  if (warps) *warps = w;
+  return wadg_ctx_set_vol_shape(a->ctx, a->curved, w, best < n ? cr[best] : 0);
 }
 
 int wadg_app_time_stage(wadg_app *a, double dt, int nstages, float *ms) {

@@ -107,6 +107,16 @@ void wadg_ctx_set_overlap(wadg_ctx *c, bool on) { c->overlap = on; }
 cudaStream_t wadg_ctx_stream(const wadg_ctx *c) { return c ? c->stream : nullptr; }
 
 namespace wadg_internal {
+int vol_automatic(const wadg_ctx *ctx, int curved, int K) {
+  wadg_ctx plain = *ctx;  // no shape selected
+  plain.vol_warps = plain.vol_rows = 0;
+  const wadg_ctx *c = &plain;
+  if (curved) {
+    WADG_DISPATCH(c, return (small_mesh<D_, N_, true>(c, K)));
+  }
+  WADG_DISPATCH(c, return (small_mesh<D_, N_, false>(c, K)));
+}
+
 // The ensemble's stage kernels over work lists (wadg_ensemble.cu): the volume
 // + surface kernel over the volume batches blist[0 .. *nb) (ascending batch
 // indices of elems_per_batch(WADG_KERNEL_VOLSURF) elements), then the update

@@ -60,6 +60,10 @@ int update_list(const wadg_ctx *c, int K, int curved, const double *Jq, const do
                 const double *VfPq, double fa, double fb, const double *dtK, double *rhsQ,
                 double *resQ, double *Q, double *Qf, const int *glist, const int *ng);
 
+// whether the volume kernel's automatic shape for K elements (vol_warps = 0) is none of
+// wadg_vol_shapes (1; wadg_capi.cu)
+int vol_automatic(const wadg_ctx *c, int curved, int K);
+
 // launch shape (elements per batch, CTAs) of the adjoint's pair VJP kernel
 // for K elements (wadg_adjoint.cu)
 int adj_pairs_shape(int dim, int N, bool curved, int K, int *E, int *grid);

@@ -10,7 +10,8 @@ are rejected, and an autotuned app still matches the reference's time step to
 import numpy as np
 import pytest
 
-from scratch_wadge_b200 import capi
+from scratch_wadge_b200 import capi, ic as IC, mesh as M
+from scratch_wadge_b200.geometry_gpu import build_geometry_gpu
 from tests.helpers import RTOL, Case, golden_names, rel
 from tests.test_gpu_parity import Dev
 
@@ -84,3 +85,36 @@ def test_autotuned_app_matches_reference_step(cuda, name):
     app.set_state(st["Q"], st["rhsQ"], st["Qf"], st["resQ"])
     app.rk_run(c.dt, 1, graph=True)
     assert rel(app.get_state()["Q"], c.z["step_Q"]) < RTOL
+
+
+@pytest.mark.parametrize("variant", ["three_kernels", "volsurf"])
+@pytest.mark.parametrize("dim,N,curved,small,large", [(2, 3, False, (32, 32), (128, 128)),
+                                                      (2, 4, True, (37, 29), (128, 64)),
+                                                      (3, 2, False, 3, 12), (3, 4, True, 4, 8)])
+def test_autotuned_app_is_not_slower_than_an_untuned_one(cuda, dim, N, curved, small, large, variant):
+    """On a small mesh the automatic shape (a warp per face of an element group,
+    up to 1.4 times as fast as the numbered ones) is one that no number selects:
+    the autotuner must time it too.  Its choice may be 5 % slower by the noise of
+    its timing, and this one's by another 5 %.  A large mesh has no shape of its own."""
+    for size in (small, large):
+        mesh = M.periodic_square(*size) if dim == 2 else M.periodic_cube(size)
+        geo = build_geometry_gpu(mesh, N)
+        app = capi.App(geo, curved)
+        app.set_stage_variant(variant)
+        kind = "vortex" if dim == 2 else "taylor_green"
+        Q, rhsQ, Qf, resQ = IC.stage0(geo, IC.initial_state(geo, kind))
+        dt = IC.time_step(geo, 0.1, N, wave_speed=IC.max_wave_speed(Q))[0]
+        app.set_state(Q, rhsQ, Qf, resQ)
+        w, times = app.autotune(dt, nstages=20)
+        assert min(times.values()) == times[w]
+        chosen = app.vol_shape()
+        assert (w == "0") == (chosen == (0, 0)) and (size == small or w != "0"), (w, chosen)
+        ms = {chosen: [], (0, 0): []}
+        for _ in range(6):
+            for shape in ms:
+                app.set_vol_shape(*shape)
+                app.set_state(Q, rhsQ, Qf, resQ)
+                time = app.time_volsurf if variant == "volsurf" else app.time_kernels
+                ms[shape].append(time(dt, 20)[0])
+        assert min(ms[chosen]) < 1.1 * min(ms[0, 0]), (size, w, times, ms)
+        app.close()
