@@ -170,13 +170,15 @@ template <int DIM, int N, bool CURVED>
 constexpr int faces_warps() {
   return VolTile<DIM, N>::H < Elem<DIM, N>::Nfaces ? Elem<DIM, N>::Nfaces : 0;
 }
+template <int DIM, int N>
+int slices_per_sm(int K) {
+  const int slices = (K + VolTile<DIM, N>::G - 1) / VolTile<DIM, N>::G;
+  return (slices + num_sms() - 1) / num_sms();
+}
 template <int DIM, int N, bool CURVED>
 bool small_mesh(const wadg_ctx *c, int K) {
   if (faces_warps<DIM, N, CURVED>() == 0 || c->vol_warps || c->vol_rows) return false;
-  constexpr int groups = 12 / Elem<DIM, N>::Nfaces;
-  const int slices = (K + VolTile<DIM, N>::G - 1) / VolTile<DIM, N>::G;
-  const int per_sm = (slices + num_sms() - 1) / num_sms();
-  return per_sm <= groups;
+  return slices_per_sm<DIM, N>(K) <= 12 / Elem<DIM, N>::Nfaces;
 }
 
 // Warps per CTA of the default map: the context's choice, else the default (0), or 16
@@ -220,6 +222,19 @@ int launch_vol_pairs_w(const wadg_ctx *c, int K, const double *vgeo, const doubl
   return after_launch(SURF ? "volume + surface kernel" : "volume kernel");
 }
 
+// The CTA of a small mesh: with two slices per SM the warps of two, so that other
+// streams' CTAs fit beside it (three or four slices take all 12; with one, a CTA of its
+// own warps alone loads the tables 0.5-1 us slower and, launched ahead, stacks on few SMs:
+// 750 tets N=2 0.60 -> 0.73 ms for 10 time steps).  Solves of 2048 triangles N=3 on
+// streams of their own, us per time step of all, 12 warps -> 6: one 82 -> 82, two 111 ->
+// 95, four 161 -> 125, eight 318 -> 221; 1296 tets N=2, 12 -> 8: one 90 -> 90, four 187 -> 162
+template <int DIM, int N, bool CURVED, bool SURF, int HH, class... A>
+int launch_vol_faces(const wadg_ctx *c, int K, A... args) {
+  if (slices_per_sm<DIM, N>(K) == 2)
+    return launch_vol_pairs_w<DIM, N, CURVED, 2 * HH, SURF, 0, HH>(c, K, args...);
+  return launch_vol_pairs_w<DIM, N, CURVED, 12, SURF, 0, HH>(c, K, args...);
+}
+
 // the volume + surface kernel in the context's CTA shape (wadg_ctx_set_vol_warps)
 template <int DIM, int N, bool CURVED>
 int launch_volsurf(const wadg_ctx *c, int K, const double *vgeo, const double *vfgeo,
@@ -230,7 +245,7 @@ int launch_volsurf(const wadg_ctx *c, int K, const double *vgeo, const double *v
   constexpr int HH = faces_warps<DIM, N, CURVED>();
   if constexpr (HH > 0)
     if (small_mesh<DIM, N, CURVED>(c, K))
-      return launch_vol_pairs_w<DIM, N, CURVED, 12, true, 0, HH>(
+      return launch_vol_faces<DIM, N, CURVED, true, HH>(
           c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, nullptr, fgeo, mapPq,
           blist, nb);
   constexpr int A0 = alt_rows<DIM, N, CURVED, 0>(), A1 = alt_rows<DIM, N, CURVED, 1>();
@@ -268,8 +283,10 @@ int launch_vol_pairs(const wadg_ctx *c, int K, const double *vgeo, const double 
   constexpr int HH = faces_warps<DIM, N, CURVED>();
   if constexpr (HH > 0)
     if (small_mesh<DIM, N, CURVED>(c, K))
-      return launch_vol_pairs_w<DIM, N, CURVED, 12, false, 0, HH>(
-          c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, rhsQf);
+      return launch_vol_faces<DIM, N, CURVED, false, HH>(c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq,
+                                                         VqLq, VfPq, Qf, rhsQ, rhsQf, (const double *)nullptr,
+                                                         (const uint32_t *)nullptr, (const int *)nullptr,
+                                                         (const int *)nullptr);
   constexpr int A0 = alt_rows<DIM, N, CURVED, 0>(), A1 = alt_rows<DIM, N, CURVED, 1>();
   if constexpr (A0 > 0)
     if (c->vol_rows == A0)

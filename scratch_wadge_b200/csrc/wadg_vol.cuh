@@ -90,7 +90,10 @@ struct VolPairsCfg {
   using T = VolTile<DIM, N, RR, HH>;
   static constexpr int H = T::H;                      // warps per element group
   static constexpr int threads = 32 * W;
-  static constexpr int E = (W / H) * T::G;            // elements per batch
+  static constexpr int E = (W / H) * T::G;            // elements of a CTA's groups
+  // elements per batch of a work list (with a warp per face the CTA's warps follow the
+  // mesh's size, the batch does not)
+  static constexpr int EB = HH ? 12 / HH * T::G : E;
   // one direction per block and the sums of the header comment
   static constexpr bool SPLIT = !CURVED && T::FACES;
   // an element's state block (doubles; [2]: double2): logarithms [2][NN] |
@@ -838,7 +841,7 @@ struct VolPairs {
 // them into its rows; rhsQ <- the whole right-hand side the surface kernel
 // would leave, rhsQf is not written (fgeo and mapPq unused when false)
 template <int DIM, int N, bool CURVED, int W, bool SURF = false, int RR = 0, int HH = 0>
-__global__ void __launch_bounds__(32 * W, 1)
+__global__ void __launch_bounds__(HH ? 384 : 32 * W, 1)  // (with a warp per face: 168 registers at any W)
 vol_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restrict__ vfgeo,
                  const double *__restrict__ nrJ, const double *__restrict__ nsJ,
                  const double *__restrict__ ntJ, const double *__restrict__ Drq,
@@ -849,7 +852,7 @@ vol_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
                  const uint32_t *__restrict__ mapPq = nullptr,
                  const int *__restrict__ blist = nullptr, const int *__restrict__ nblist = nullptr) {
   using V = VolPairs<DIM, N, CURVED, W, RR, HH>;
-  constexpr int Nq = V::Nq, NF = V::NF, Nf = V::Nf, R = V::R, L = V::L, E = V::E, H = V::H;
+  constexpr int Nq = V::Nq, NF = V::NF, Nf = V::Nf, R = V::R, L = V::L, E = V::C::EB, H = V::H;
   extern __shared__ double smem[];
   V v(smem);
   constexpr bool PRE = V::C::PREFETCH;
@@ -894,14 +897,14 @@ vol_pairs_kernel(int K, const double *__restrict__ vgeo, const double *__restric
   // The work: batches of E elements, all of them or (a work list: the
   // ensemble's active instances) the ascending batch indices blist[0 ..
   // *nblist), each cut into its NG group slices of G elements.  The groups
-  // take the slices independently: in round i group q of CTA b takes slice
-  // (i NG + q) grid + b, so a last, partial round leaves the busy groups
+  // take the slices independently: in round i group q of CTA b (of W / H) takes
+  // slice (i W / H + q) grid + b, so a last, partial round leaves the busy groups
   // spread over every SM (rather than whole CTAs busy and the other SMs
   // idle).  Every slice is G consecutive elements, so the elements that
   // share a warp, and the results, do not depend on the schedule.
-  constexpr int NG = W / H;
+  constexpr int NG = E / G;
   const int nb = blist ? *nblist : (K + E - 1) / E;
-  const int ns = nb * NG, sstep = (int)gridDim.x * NG;
+  const int ns = nb * NG, sstep = (int)gridDim.x * (W / H);
   auto slice = [&](int g) {  // first element of slice g (K past the end)
     if (g >= ns) return K;
     const int cb = g / NG;

@@ -262,6 +262,42 @@ def test_small_mesh_shape_edges(cuda, dim, N, curved):
 
 
 @pytest.mark.parametrize("dim,N,curved", CASES)
+def test_small_mesh_cta_sizes(cuda, dim, N, curved):
+    """A small mesh's CTA has 12 warps, or those of two slices where an SM has
+    two: the element counts on either side of one and of two slices per SM give
+    the same elements the same bits, and those of the reference's kernels."""
+    ctx = capi.Context(R.load(dim, N))
+    G = ctx.shape("volsurf", curved, 1)[0] // (12 // (dim + 1))
+    one = G * torch.cuda.get_device_properties(0).multi_processor_count
+    geo = build_geometry_gpu(mesh_with_at_least(dim, curved, 2 * one + 1), N)
+    d = Dev(cuda, geo, curved)
+    ref = oracle(geo.ops, curved)
+    st = state(geo, curved, 9)
+    want = {k: v.copy() for k, v in st.items()}
+    ref.vol(geo, want["Qf"], want["rhsQ"], want["rhsQf"])
+    faces = want["rhsQf"].copy()
+    ref.surf(geo, want["Qf"], want["rhsQf"], want["rhsQ"])
+    p = lambda s, *names: [s[n].data_ptr() for n in names]
+    geom = ("vgeo", "vfgeo", "nrJ", "nsJ", "ntJ", "Drq", "Dsq", "Dtq", "VqLq", "VfPq")
+    got = {}
+    for K in (one - 1, one, one + 1, 2 * one - G, 2 * one, 2 * one + 1):
+        s = d.put(st)
+        d.ctx.vol(curved, K, *p(d.g, *geom), *p(s, "Qf", "rhsQ", "rhsQf"))
+        d.sync()
+        f = d.get(s)["rhsQf"]
+        s = d.put(st)
+        d.ctx.volsurf(curved, K, *p(d.g, "vgeo", "vfgeo", "fgeo", "mapPq", *geom[2:]), *p(s, "Qf", "rhsQ"))
+        d.sync()
+        r = d.get(s)["rhsQ"]
+        assert rel(f[:K], faces[:K]) < RTOL and rel(r[:K], want["rhsQ"][:K]) < RTOL, K
+        assert (f[K:] == SENTINEL).all() and np.array_equal(r[K:], st["rhsQ"][K:]), K
+        got[K] = (f, r)
+    whole = one - one % G - G  # slices that every count has whole
+    for f, r in got.values():
+        assert np.array_equal(f[:whole], got[one][0][:whole]) and np.array_equal(r[:whole], got[one][1][:whole])
+
+
+@pytest.mark.parametrize("dim,N,curved", CASES)
 def test_update_shape_edges(cuda, dim, N, curved):
     """The update kernel's two shapes (a warp per m-tile of the output projection
     on meshes of few groups): a single element, a partial group, and the last
