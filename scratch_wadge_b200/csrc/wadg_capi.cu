@@ -273,6 +273,13 @@ int wadg_vol_warps_candidates(const wadg_ctx *ctx, int curved, int *out) {
   }
 }
 
+static int vol_more(const wadg_ctx *c, int curved, int *out) {
+  if (curved) {
+    WADG_DISPATCH(c, return (vol_warps_more<D_, N_, true>(out)));
+  }
+  WADG_DISPATCH(c, return (vol_warps_more<D_, N_, false>(out)));
+}
+
 int wadg_ctx_set_vol_warps(wadg_ctx *ctx, int curved, int warps) {
   if (!ctx) return fail(WADG_ERR_INVALID, "null context");
   if (warps != 0) {
@@ -280,6 +287,8 @@ int wadg_ctx_set_vol_warps(wadg_ctx *ctx, int curved, int warps) {
     const int n = wadg_vol_warps_candidates(ctx, curved, cand);
     bool ok = false;
     for (int i = 0; i < n; ++i) ok = ok || cand[i] == warps;
+    const int m = vol_more(ctx, curved, cand);
+    for (int i = 0; i < m; ++i) ok = ok || cand[i] == warps;
     if (!ok) return fail(WADG_ERR_INVALID, "%d warps per CTA is not a compiled shape", warps);
   }
   ctx->vol_warps = warps;

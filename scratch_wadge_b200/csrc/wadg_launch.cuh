@@ -114,6 +114,14 @@ constexpr int volpairsW_cand(int i) {
   return i == 0 ? W0 : (W0 - 2 * i >= 2 ? W0 - 2 * i : 0);
 }
 
+// More counts of warps that wadg_ctx_set_vol_warps takes, though they are no candidates:
+// they were, while an element took more shared memory
+template <int DIM, int N, bool CURVED>
+constexpr int volpairsW_more(int i) {
+  if (DIM == 3 && CURVED && N <= 2) return i == 0 ? 6 : N == 2 ? 4 : 0;
+  return DIM == 2 && N == 1 && !CURVED && i == 0 ? 10 : 0;
+}
+
 // The other node-to-thread maps: half and twice the default's lanes per
 // element (about twice and half its rows per lane), each given to the kernels
 // as RR = rows per lane.  A map is a candidate when it has as many lanes as
@@ -187,7 +195,8 @@ bool small_mesh(const wadg_ctx *c, int K) {
 // warps, by slices per SM: N=3 (6 groups for 8) 6.9 1.318 -> 1.223, 13.8 2.10 ->
 // 2.02; curved N=3 6.9 1.58 -> 1.44; N=2 13.8 2.31 -> 2.17; curved N=2 6.9 1.70 ->
 // 1.53; curved N=4 (12 groups for 16) 12.2 2.05 -> 1.83, affine N=4 13.8 (not
-// taken) 1.79 -> 1.81.  Same bits
+// taken) 1.79 -> 1.81; volume + surface kernel, us, N=1 6.5 23.8 -> 19.6, 7.4 24.3 -> 21.4,
+// 13.0 33.7 -> 30.2.  Same bits
 template <int DIM, int N, bool CURVED>
 int default_warps(const wadg_ctx *c, int K) {
   constexpr int W0 = volpairsW<DIM, N, CURVED>(), W1 = volpairsW_cand<DIM, N, CURVED>(1);
@@ -196,6 +205,41 @@ int default_warps(const wadg_ctx *c, int K) {
   const int slices = (K + VolTile<DIM, N>::G - 1) / VolTile<DIM, N>::G;
   const int m = (slices + num_sms() - 1) / num_sms();
   return m <= 2 * g1 && (m + g1 - 1) / g1 < (m + g0 - 1) / g0 ? W1 : 0;
+}
+
+// The CTA of a small mesh: with two slices per SM the warps of two, so that other
+// streams' CTAs fit beside it (three or four slices take all 12; with one, a CTA of its
+// own warps alone loads the tables 0.5-1 us slower and, launched ahead, stacks on few SMs:
+// 750 tets N=2 0.60 -> 0.73 ms for 10 time steps).  Solves of 2048 triangles N=3 on
+// streams of their own, us per time step of all, 12 warps -> 6: one 82 -> 82, two 111 ->
+// 95, four 161 -> 125, eight 318 -> 221; 1296 tets N=2, 12 -> 8: one 90 -> 90, four 187 -> 162
+template <int W_, int RR_ = 0, int HH_ = 0>
+struct VolShape {
+  static constexpr int W = W_, RR = RR_, HH = HH_;
+};
+
+// f(VolShape) with the shape of the volume kernels for K elements: the context's
+// (wadg_ctx_set_vol_shape), else the automatic one
+template <int DIM, int N, bool CURVED, class F>
+int with_vol_shape(const wadg_ctx *c, int K, F f) {
+  constexpr int HH = faces_warps<DIM, N, CURVED>();
+  if constexpr (HH > 0)
+    if (small_mesh<DIM, N, CURVED>(c, K))
+      return slices_per_sm<DIM, N>(K) == 2 ? f(VolShape<2 * HH, 0, HH>()) : f(VolShape<12, 0, HH>());
+  constexpr int A0 = alt_rows<DIM, N, CURVED, 0>(), A1 = alt_rows<DIM, N, CURVED, 1>();
+  if constexpr (A0 > 0)
+    if (c->vol_rows == A0) return f(VolShape<alt_warps<DIM, N, CURVED, A0>(), A0>());
+  if constexpr (A1 > 0)
+    if (c->vol_rows == A1) return f(VolShape<alt_warps<DIM, N, CURVED, A1>(), A1>());
+  constexpr int W0 = volpairsW<DIM, N, CURVED>();
+  constexpr int W1 = volpairsW_cand<DIM, N, CURVED>(1), W2 = volpairsW_cand<DIM, N, CURVED>(2);
+  constexpr int W3 = volpairsW_more<DIM, N, CURVED>(0), W4 = volpairsW_more<DIM, N, CURVED>(1);
+  const int warps = default_warps<DIM, N, CURVED>(c, K);
+  if (W1 && warps == W1) return f(VolShape<(W1 ? W1 : W0)>());
+  if (W2 && warps == W2) return f(VolShape<(W2 ? W2 : W0)>());
+  if (W3 && warps == W3) return f(VolShape<(W3 ? W3 : W0)>());
+  if (W4 && warps == W4) return f(VolShape<(W4 ? W4 : W0)>());
+  return f(VolShape<W0>());
 }
 
 // SURF: the volume + surface kernel (rhsQf unused; fgeo, mapPq read)
@@ -222,90 +266,37 @@ int launch_vol_pairs_w(const wadg_ctx *c, int K, const double *vgeo, const doubl
   return after_launch(SURF ? "volume + surface kernel" : "volume kernel");
 }
 
-// The CTA of a small mesh: with two slices per SM the warps of two, so that other
-// streams' CTAs fit beside it (three or four slices take all 12; with one, a CTA of its
-// own warps alone loads the tables 0.5-1 us slower and, launched ahead, stacks on few SMs:
-// 750 tets N=2 0.60 -> 0.73 ms for 10 time steps).  Solves of 2048 triangles N=3 on
-// streams of their own, us per time step of all, 12 warps -> 6: one 82 -> 82, two 111 ->
-// 95, four 161 -> 125, eight 318 -> 221; 1296 tets N=2, 12 -> 8: one 90 -> 90, four 187 -> 162
-template <int DIM, int N, bool CURVED, bool SURF, int HH, class... A>
-int launch_vol_faces(const wadg_ctx *c, int K, A... args) {
-  if (slices_per_sm<DIM, N>(K) == 2)
-    return launch_vol_pairs_w<DIM, N, CURVED, 2 * HH, SURF, 0, HH>(c, K, args...);
-  return launch_vol_pairs_w<DIM, N, CURVED, 12, SURF, 0, HH>(c, K, args...);
-}
-
-// the volume + surface kernel in the context's CTA shape (wadg_ctx_set_vol_warps)
 template <int DIM, int N, bool CURVED>
 int launch_volsurf(const wadg_ctx *c, int K, const double *vgeo, const double *vfgeo,
                    const double *fgeo, const uint32_t *mapPq, const double *nrJ,
                    const double *nsJ, const double *ntJ, const double *Drq, const double *Dsq,
                    const double *Dtq, const double *VqLq, const double *VfPq, const double *Qf,
                    double *rhsQ, const int *blist = nullptr, const int *nb = nullptr) {
-  constexpr int HH = faces_warps<DIM, N, CURVED>();
-  if constexpr (HH > 0)
-    if (small_mesh<DIM, N, CURVED>(c, K))
-      return launch_vol_faces<DIM, N, CURVED, true, HH>(
-          c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, nullptr, fgeo, mapPq,
-          blist, nb);
-  constexpr int A0 = alt_rows<DIM, N, CURVED, 0>(), A1 = alt_rows<DIM, N, CURVED, 1>();
-  if constexpr (A0 > 0)
-    if (c->vol_rows == A0)
-      return launch_vol_pairs_w<DIM, N, CURVED, alt_warps<DIM, N, CURVED, A0>(), true, A0>(
-          c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, nullptr, fgeo,
-          mapPq, blist, nb);
-  if constexpr (A1 > 0)
-    if (c->vol_rows == A1)
-      return launch_vol_pairs_w<DIM, N, CURVED, alt_warps<DIM, N, CURVED, A1>(), true, A1>(
-          c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, nullptr, fgeo,
-          mapPq, blist, nb);
-  constexpr int W1 = volpairsW_cand<DIM, N, CURVED>(1), W2 = volpairsW_cand<DIM, N, CURVED>(2);
-  const int warps = default_warps<DIM, N, CURVED>(c, K);
-  if (W1 && warps == W1)
-    return launch_vol_pairs_w<DIM, N, CURVED, (W1 ? W1 : 2), true>(
-        c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, nullptr, fgeo, mapPq,
-        blist, nb);
-  if (W2 && warps == W2)
-    return launch_vol_pairs_w<DIM, N, CURVED, (W2 ? W2 : 2), true>(
-        c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, nullptr, fgeo, mapPq,
-        blist, nb);
-  return launch_vol_pairs_w<DIM, N, CURVED, volpairsW<DIM, N, CURVED>(), true>(
-      c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, nullptr, fgeo, mapPq,
-      blist, nb);
+  return with_vol_shape<DIM, N, CURVED>(c, K, [&](auto s) {
+    using S = decltype(s);
+    return launch_vol_pairs_w<DIM, N, CURVED, S::W, true, S::RR, S::HH>(
+        c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, nullptr, fgeo, mapPq, blist, nb);
+  });
 }
 
-// the context's CTA shape (wadg_ctx_set_vol_warps), else the default
 template <int DIM, int N, bool CURVED>
 int launch_vol_pairs(const wadg_ctx *c, int K, const double *vgeo, const double *vfgeo,
                      const double *nrJ, const double *nsJ, const double *ntJ, const double *Drq,
                      const double *Dsq, const double *Dtq, const double *VqLq, const double *VfPq,
                      const double *Qf, double *rhsQ, double *rhsQf) {
-  constexpr int HH = faces_warps<DIM, N, CURVED>();
-  if constexpr (HH > 0)
-    if (small_mesh<DIM, N, CURVED>(c, K))
-      return launch_vol_faces<DIM, N, CURVED, false, HH>(c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq,
-                                                         VqLq, VfPq, Qf, rhsQ, rhsQf, (const double *)nullptr,
-                                                         (const uint32_t *)nullptr, (const int *)nullptr,
-                                                         (const int *)nullptr);
-  constexpr int A0 = alt_rows<DIM, N, CURVED, 0>(), A1 = alt_rows<DIM, N, CURVED, 1>();
-  if constexpr (A0 > 0)
-    if (c->vol_rows == A0)
-      return launch_vol_pairs_w<DIM, N, CURVED, alt_warps<DIM, N, CURVED, A0>(), false, A0>(
-          c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, rhsQf);
-  if constexpr (A1 > 0)
-    if (c->vol_rows == A1)
-      return launch_vol_pairs_w<DIM, N, CURVED, alt_warps<DIM, N, CURVED, A1>(), false, A1>(
-          c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, rhsQf);
-  constexpr int W1 = volpairsW_cand<DIM, N, CURVED>(1), W2 = volpairsW_cand<DIM, N, CURVED>(2);
-  const int warps = default_warps<DIM, N, CURVED>(c, K);
-  if (W1 && warps == W1)
-    return launch_vol_pairs_w<DIM, N, CURVED, (W1 ? W1 : 2)>(c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq,
-                                                             Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, rhsQf);
-  if (W2 && warps == W2)
-    return launch_vol_pairs_w<DIM, N, CURVED, (W2 ? W2 : 2)>(c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq,
-                                                             Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, rhsQf);
-  return launch_vol_pairs_w<DIM, N, CURVED, volpairsW<DIM, N, CURVED>()>(
-      c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, rhsQf);
+  return with_vol_shape<DIM, N, CURVED>(c, K, [&](auto s) {
+    using S = decltype(s);
+    return launch_vol_pairs_w<DIM, N, CURVED, S::W, false, S::RR, S::HH>(
+        c, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq, Qf, rhsQ, rhsQf);
+  });
+}
+
+template <int DIM, int N, bool CURVED>
+int vol_warps_more(int *out) {
+  int n = 0;
+  for (int i = 0; i < 2; ++i)
+    if (int w = volpairsW_more<DIM, N, CURVED>(i)) out[n++] = w;
+  return n;
 }
 
 template <int DIM, int N, bool CURVED>
@@ -390,37 +381,18 @@ int update_grid(int K, int *grid) {
 }
 
 // the launch shape of one kernel for K elements (wadg_kernel_shape)
-template <int DIM, int N, bool CURVED, int W, int RR = 0, int HH = 0>
-void vol_shape(int K, int *E, int *grid) {
-  using C = VolPairsCfg<DIM, N, CURVED, W, RR, HH>;
-  *E = C::E;
-  *grid = vol_grid<C>(K);
-}
-
 template <int DIM, int N, bool CURVED>
 int kernel_shape(const wadg_ctx *c, int kernel, int K, int *E, int *grid) {
-  constexpr int W1 = volpairsW_cand<DIM, N, CURVED>(1), W2 = volpairsW_cand<DIM, N, CURVED>(2);
-  constexpr int A0 = alt_rows<DIM, N, CURVED, 0>(), A1 = alt_rows<DIM, N, CURVED, 1>();
-  if ((kernel == WADG_KERNEL_VOL || kernel == WADG_KERNEL_VOLSURF) && c->vol_rows) {
-    if constexpr (A0 > 0)
-      if (c->vol_rows == A0) vol_shape<DIM, N, CURVED, alt_warps<DIM, N, CURVED, A0>(), A0>(K, E, grid);
-    if constexpr (A1 > 0)
-      if (c->vol_rows == A1) vol_shape<DIM, N, CURVED, alt_warps<DIM, N, CURVED, A1>(), A1>(K, E, grid);
-    return WADG_OK;
-  }
-  constexpr int HH = faces_warps<DIM, N, CURVED>();
-  if constexpr (HH > 0)
-    if ((kernel == WADG_KERNEL_VOL || kernel == WADG_KERNEL_VOLSURF) && small_mesh<DIM, N, CURVED>(c, K)) {
-      vol_shape<DIM, N, CURVED, 12, 0, HH>(K, E, grid);
-      return WADG_OK;
-    }
-  const int warps = default_warps<DIM, N, CURVED>(c, K);
   switch (kernel) {
     case WADG_KERNEL_VOL:
-      if (W1 && warps == W1) vol_shape<DIM, N, CURVED, (W1 ? W1 : 2)>(K, E, grid);
-      else if (W2 && warps == W2) vol_shape<DIM, N, CURVED, (W2 ? W2 : 2)>(K, E, grid);
-      else vol_shape<DIM, N, CURVED, volpairsW<DIM, N, CURVED>()>(K, E, grid);
-      return WADG_OK;
+    case WADG_KERNEL_VOLSURF:
+      return with_vol_shape<DIM, N, CURVED>(c, K, [&](auto s) {
+        using S = decltype(s);
+        using C = VolPairsCfg<DIM, N, CURVED, S::W, S::RR, S::HH>;
+        *E = C::EB;
+        *grid = vol_grid<C>(K);
+        return (int)WADG_OK;
+      });
     case WADG_KERNEL_SURF:
       *E = SurfMmaCfg<DIM, N>::EW;
       *grid = (K + *E - 1) / *E;
@@ -428,11 +400,6 @@ int kernel_shape(const wadg_ctx *c, int kernel, int K, int *E, int *grid) {
     case WADG_KERNEL_UPDATE:
       *E = UpdMmaCfg<DIM, N, CURVED>::EW;
       return update_grid<DIM, N, CURVED>(K, grid);
-    case WADG_KERNEL_VOLSURF:  // the same CTA shapes as the volume kernel
-      if (W1 && warps == W1) vol_shape<DIM, N, CURVED, (W1 ? W1 : 2)>(K, E, grid);
-      else if (W2 && warps == W2) vol_shape<DIM, N, CURVED, (W2 ? W2 : 2)>(K, E, grid);
-      else vol_shape<DIM, N, CURVED, volpairsW<DIM, N, CURVED>()>(K, E, grid);
-      return WADG_OK;
     case WADG_KERNEL_ADJ_PAIRS:
       return wadg_internal::adj_pairs_shape(DIM, N, CURVED, K, E, grid);
     case WADG_KERNEL_STAGE: {

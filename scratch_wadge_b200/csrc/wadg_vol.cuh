@@ -117,8 +117,10 @@ struct VolPairsCfg {
   static constexpr int SE = up(mx(nS, 3 * El::Nfields * El::Nq), mL < 8 ? 2 * mL : 8);
   // face-row accumulators: SPLIT [2][NF] (sum F0, sum pa), (m0, m1), 3D (m2, E), 2D E [NF];
   // else the Nfields rows [NF]
-  static constexpr int SA = SPLIT ? up((DIM == 3 ? 6 : 5) * El::NfqNf, mL < 8 ? 2 * mL : 8)
-                                  : up(El::Nfields * El::NfqNf, mL);
+  static constexpr int nA = (DIM == 3 ? 6 : 5) * El::NfqNf;
+  // (-2 mod 16 serves L = 1 as well as 2, and 16 warps of 2D N=1 fit with it)
+  static constexpr int SA = !SPLIT ? up(El::Nfields * El::NfqNf, mL)
+                            : T::L == 1 && nA % 16 == 14 ? nA : up(nA, mL < 8 ? 2 * mL : 8);
   // per-face nJ and G (affine), and the next slice's G
   static constexpr int SN = CURVED ? 0 : El::Nfaces * DIM + 2 * El::Nvgeo;
   static constexpr int nD = DIM * El::Nq * El::Nq;

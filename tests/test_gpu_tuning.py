@@ -63,6 +63,31 @@ def test_node_to_thread_maps_where_compiled(cuda):
     assert all(r == 0 for _, r in d3.ctx.vol_shapes(c3.curved))
 
 
+@pytest.mark.parametrize("dim,N,curved,warps", [(2, 1, False, 16), (2, 1, False, 10), (3, 1, True, 6),
+                                                (3, 2, True, 6), (3, 2, True, 4)])
+def test_counts_that_were_candidates_once_are_still_taken(cuda, dim, N, curved, warps):
+    """A count of warps that an earlier form's shared memory made a candidate is
+    still accepted, runs at that count and gives the default map's bits."""
+    geo = build_geometry_gpu(M.periodic_square(20, 16) if dim == 2 else
+                             M.periodic_cube(5, warp=M.warp_cube(0.05)), N)
+    d = Dev(cuda, geo, curved)
+    kind = "vortex" if dim == 2 else "density_wave"
+    Q, rhsQ, Qf, resQ = IC.stage0(geo, IC.initial_state(geo, kind))
+    got = []
+    for w in (d.ctx.vol_warps_candidates(curved)[0], warps):
+        d.ctx.set_vol_warps(curved, w)
+        assert capi.lib().wadg_ctx_get_vol_warps(d.ctx.h) == w
+        got.append([d.ctx.shape("vol", curved, geo.K)[0]])
+        for run in (d.vol, d.volsurf):
+            s = d.put(dict(rhsQ=rhsQ, Qf=Qf, rhsQf=np.zeros_like(Qf)))
+            run(s)
+            d.sync()
+            got[-1].append(d.get(s))
+    assert got[1][0] * 12 == got[0][0] * warps  # elements per batch, 12 warps at first
+    for a, b in zip(got[0][1:], got[1][1:]):
+        assert all(np.array_equal(a[k], b[k]) for k in a)
+
+
 def test_shapes_that_are_not_compiled_are_rejected(cuda):
     c = Case("tg3d_affine_N3")
     d = Dev(cuda, c.geo, c.curved)
