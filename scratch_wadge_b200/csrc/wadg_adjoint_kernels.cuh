@@ -84,10 +84,6 @@ template <int T> __device__ __forceinline__ double poly2dG(double u) {
   return fma(p, u, -0.6666666666666655);
 }
 
-template <int V> struct IntTag {
-  static constexpr int value = V;
-};
-
 // Vector-Jacobian product of the contracted two-point flux F_S(a, b).n
 // (Euler3Daffine.okl:107-148, Euler2D.okl:139-161) with the
 // adjoint c of its Nfields components: adds the adjoints of a's and b's

@@ -33,6 +33,11 @@ template <int DIM, int N> struct Elem {
   static constexpr int NN = Nq + NfqNf;   // volume + face nodes
 };
 
+// an integer constant as a function argument
+template <int V> struct IntTag {
+  static constexpr int value = V;
+};
+
 // 8-byte asynchronous global -> shared copies (cp.async, sm_80 and later):
 // the copies of a block are in flight together, occupying no registers, while
 // the issuing threads go on computing; commit + wait completes them

@@ -196,14 +196,19 @@ bool small_mesh(const wadg_ctx *c, int K) {
 // 2.02; curved N=3 6.9 1.58 -> 1.44; N=2 13.8 2.31 -> 2.17; curved N=2 6.9 1.70 ->
 // 1.53; curved N=4 (12 groups for 16) 12.2 2.05 -> 1.83, affine N=4 13.8 (not
 // taken) 1.79 -> 1.81; volume + surface kernel, us, N=1 6.5 23.8 -> 19.6, 7.4 24.3 -> 21.4,
-// 13.0 33.7 -> 30.2.  Same bits
+// 13.0 33.7 -> 30.2.  Curved 3D N=2: eight where twelve save no round (255 registers a
+// thread for 168), us, 12 -> 8 warps, smooth / random states: 3.7 29.5 -> 27.5 / 40.5 ->
+// 38.9; 6.7 48.7 -> 43.9 / 70.0 -> 65.3; 5.1 (a round against two) 34.6, 8 warps 39.1.  Same bits
 template <int DIM, int N, bool CURVED>
 int default_warps(const wadg_ctx *c, int K) {
   constexpr int W0 = volpairsW<DIM, N, CURVED>(), W1 = volpairsW_cand<DIM, N, CURVED>(1);
+  if (DIM == 3 && CURVED && N == 2 && !c->vol_warps && !c->vol_rows) {
+    const int m = slices_per_sm<DIM, N>(K), g = W0 / VolTile<DIM, N>::H, g8 = 8 / VolTile<DIM, N>::H;
+    return (m + g8 - 1) / g8 <= (m + g - 1) / g ? 8 : 0;
+  }
   if (c->vol_warps || c->vol_rows || DIM == 3 || (N == 4 && !CURVED) || W1 <= W0) return c->vol_warps;
   constexpr int g0 = W0 / VolTile<DIM, N>::H, g1 = W1 / VolTile<DIM, N>::H;
-  const int slices = (K + VolTile<DIM, N>::G - 1) / VolTile<DIM, N>::G;
-  const int m = (slices + num_sms() - 1) / num_sms();
+  const int m = slices_per_sm<DIM, N>(K);
   return m <= 2 * g1 && (m + g1 - 1) / g1 < (m + g0 - 1) / g0 ? W1 : 0;
 }
 
@@ -325,6 +330,21 @@ int vol_shapes(int *warps, int *rows) {
   return n;
 }
 
+// f(warps per CTA) of the fused stage kernel for K elements: the volume kernel's default,
+// but at curved 3D N=2 eight where twelve save no round (255 registers a thread for 168, and
+// the stage spills 80 bytes at 168).  us, 12 -> 8 warps: K=162 36.9 -> 27.7, 7986 (two
+// rounds either way) 68.2 -> 51.5; 24576 (four rounds, or six) 156 at 12
+template <int DIM, int N, bool CURVED, class F>
+int with_stage_warps(int K, F f) {
+  constexpr int W = stage_warps<DIM, N, CURVED, volpairsW<DIM, N, CURVED>()>();
+  if constexpr (DIM == 3 && CURVED && N == 2) {
+    constexpr int E = VolPairsCfg<DIM, N, CURVED, W>::E, E8 = VolPairsCfg<DIM, N, CURVED, 8>::E;
+    auto rounds = [&](int e) { return ((K + e - 1) / e + num_sms() - 1) / num_sms(); };
+    if (rounds(E8) <= rounds(E)) return f(IntTag<8>());
+  }
+  return f(IntTag<W>());
+}
+
 template <int DIM, int N, bool CURVED>
 int launch_stage(const wadg_ctx *c, int K, const double *vgeo, const double *vfgeo,
                  const double *fgeo, const uint32_t *mapPq, const double *nrJ, const double *nsJ,
@@ -333,20 +353,22 @@ int launch_stage(const wadg_ctx *c, int K, const double *vgeo, const double *vfg
                  double fa, double fb, double fdt, const double *uq, const double *uf, double *Q,
                  double *resQ, double *uq_out, double *uf_out) {
   if (uf_out == uf) return fail(WADG_ERR_INVALID, "stage: uf_out must not be uf");
-  constexpr int W = stage_warps<DIM, N, CURVED, volpairsW<DIM, N, CURVED>()>();
-  using C = VolPairsCfg<DIM, N, CURVED, W>;
-  auto kern = stage_kernel<DIM, N, CURVED, W>;
-  static wadg_internal::PerDevice<bool> attr;
-  if (!attr.here()) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem_vol);
-    if (e != cudaSuccess) return cuda_check(e, "stage kernel smem attribute");
-    attr.here() = true;
-  }
-  const int grid = persistent_grid(K, C::E, C::smem_vol);
-  kern<<<grid, C::threads, C::smem_vol, c->stream>>>(K, vgeo, vfgeo, fgeo, mapPq, nrJ, nsJ, ntJ, Drq,
-                                                  Dsq, Dtq, VqLq, VfPq, VqPq, Jq, fa, fb, fdt, uq,
-                                                  uf, Q, resQ, uq_out, uf_out, c->phys);
-  return after_launch("stage kernel");
+  return with_stage_warps<DIM, N, CURVED>(K, [&](auto w) {
+    constexpr int W = decltype(w)::value;
+    using C = VolPairsCfg<DIM, N, CURVED, W>;
+    auto kern = stage_kernel<DIM, N, CURVED, W>;
+    static wadg_internal::PerDevice<bool> attr;
+    if (!attr.here()) {
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem_vol);
+      if (e != cudaSuccess) return cuda_check(e, "stage kernel smem attribute");
+      attr.here() = true;
+    }
+    const int grid = persistent_grid(K, C::E, C::smem_vol);
+    kern<<<grid, C::threads, C::smem_vol, c->stream>>>(K, vgeo, vfgeo, fgeo, mapPq, nrJ, nsJ, ntJ, Drq,
+                                                    Dsq, Dtq, VqLq, VfPq, VqPq, Jq, fa, fb, fdt, uq,
+                                                    uf, Q, resQ, uq_out, uf_out, c->phys);
+    return after_launch("stage kernel");
+  });
 }
 
 template <int DIM, int N>
@@ -402,12 +424,13 @@ int kernel_shape(const wadg_ctx *c, int kernel, int K, int *E, int *grid) {
       return update_grid<DIM, N, CURVED>(K, grid);
     case WADG_KERNEL_ADJ_PAIRS:
       return wadg_internal::adj_pairs_shape(DIM, N, CURVED, K, E, grid);
-    case WADG_KERNEL_STAGE: {
-      using C = VolPairsCfg<DIM, N, CURVED, stage_warps<DIM, N, CURVED, volpairsW<DIM, N, CURVED>()>()>;
-      *E = C::E;
-      *grid = persistent_grid(K, C::E, C::smem_vol);
-      return WADG_OK;
-    }
+    case WADG_KERNEL_STAGE:
+      return with_stage_warps<DIM, N, CURVED>(K, [&](auto w) {
+        using C = VolPairsCfg<DIM, N, CURVED, decltype(w)::value>;
+        *E = C::E;
+        *grid = persistent_grid(K, C::E, C::smem_vol);
+        return (int)WADG_OK;
+      });
   }
   return fail(WADG_ERR_INVALID, "unknown kernel %d", kernel);
 }

@@ -261,6 +261,44 @@ def test_small_mesh_shape_edges(cuda, dim, N, curved):
         assert np.array_equal(h["rhsQ"][K:], st["rhsQ"][K:]), K
 
 
+def test_warps_by_rounds_curved_n2(cuda):
+    """At curved 3D N=2 the volume and fused stage kernels take eight warps where
+    twelve save no round: a partial batch, the last count of two rounds of eight
+    and the first past it (twelve), against the reference's stage."""
+    two = 2 * 32 * torch.cuda.get_device_properties(0).multi_processor_count
+    geo = build_geometry_gpu(mesh_with_at_least(3, True, two + 1), 2)
+    d = Dev(cuda, geo, True)
+    st = state(geo, True, 5)
+    dt = IC.time_step(geo, 0.1, 2, nsteps=1, wave_speed=IC.max_wave_speed(st["Q"]))[0]
+    ref = oracle(geo.ops, True)
+    want = _first(st, geo.K)
+    want["rhsQf"][:] = 0.0
+    ref.vol(geo, want["Qf"], want["rhsQ"], want["rhsQf"])
+    ref.surf(geo, want["Qf"].copy(), want["rhsQf"], want["rhsQ"])
+    rhs = want["rhsQ"].copy()
+    ref.update(geo, IC.RK4A[3], IC.RK4B[3], dt, want["rhsQ"], want["resQ"], want["Q"], want["Qf"])
+    names = ("vgeo", "vfgeo", "fgeo", "mapPq", "nrJ", "nsJ", "ntJ", "Drq", "Dsq", "Dtq", "VqLq", "VfPq",
+             "VqPq", "Jq")
+    for K, E in ((33, 32), (two, 32), (two + 1, 48)):
+        assert d.ctx.shape("stage", True, K)[0] == E, K
+        s = d.put(st)
+        out = {k: torch.full_like(s[k], SENTINEL) for k in ("rhsQ", "Qf")}
+        d.ctx.stage(True, K, *[d.g[n].data_ptr() for n in names], IC.RK4A[3], IC.RK4B[3], dt,
+                    *[s[k].data_ptr() for k in ("rhsQ", "Qf", "Q", "resQ")], out["rhsQ"].data_ptr(),
+                    out["Qf"].data_ptr())
+        d.sync()
+        h = d.get(dict(s, **out))
+        for k in ("Q", "rhsQ", "Qf", "resQ"):
+            assert rel(h[k][:K], want[k][:K]) < RTOL, (K, k, rel(h[k][:K], want[k][:K]))
+        assert np.array_equal(h["Q"][K:], st["Q"][K:]) and (h["rhsQ"][K:] == SENTINEL).all(), K
+        assert K == 33 or d.ctx.shape("volsurf", True, K)[0] == E, K
+        s = d.put(st)
+        d.ctx.volsurf(True, K, *[d.g[n].data_ptr() for n in names[:12]], s["Qf"].data_ptr(), s["rhsQ"].data_ptr())
+        d.sync()
+        h = d.get(s)
+        assert rel(h["rhsQ"][:K], rhs[:K]) < RTOL and np.array_equal(h["rhsQ"][K:], st["rhsQ"][K:]), K
+
+
 @pytest.mark.parametrize("dim,N,curved", CASES)
 def test_small_mesh_cta_sizes(cuda, dim, N, curved):
     """A small mesh's CTA has 12 warps, or those of two slices where an SM has
