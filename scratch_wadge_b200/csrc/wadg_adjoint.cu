@@ -88,7 +88,9 @@ constexpr int adjW() {
   constexpr size_t w = (227 * 1024 - C1::fixed) / per_warp;
   // 12 (168 registers per thread) or at most 8 (255): 10 would leave them 168 for
   // less work, and three rows per lane in 3D need about 250.  Below 8, six warps
-  // where they hold 12 elements, else 4 (curved 3D N=4: six were not measured)
+  // where they hold 12 elements, else 4 (curved 3D N=4, reverse sweep of 10 steps, ms, 4 / 6
+  // warps: K=162 3.56 / 4.38, 750 5.77 / 5.16, 1296 8.23 / 8.33, 2058 11.30 / 11.69, 4374
+  // 21.4 / 21.9)
   constexpr int cap = DIM == 3 && VolTile<DIM, N>::R >= 3 ? 8 : 12;
   constexpr int wc = w >= 12 && cap == 12 ? 12 : w >= 8 ? 8 : w >= 6 && VolTile<DIM, N>::G >= 4 ? 6 : w >= 4 ? 4 : (int)w;
   return wc < H ? H : (wc / H) * H;
