@@ -63,9 +63,11 @@ bool overlaps(const wadg_ctx *c, int K) {
   return c->overlap && K <= VolTile<DIM, N>::G * num_sms();
 }
 
-// a kernel on the context's stream
+// a kernel on the context's stream.  The error of a failed launch is taken off the
+// runtime's record: left there, it would be the next call's
 template <class... KA, class... A>
-int launch(const wadg_ctx *c, bool overlap, void (*kern)(KA...), int grid, int threads, size_t smem, A... args) {
+int launch(const wadg_ctx *c, const char *name, bool overlap, void (*kern)(KA...), int grid, int threads,
+           size_t smem, A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)threads);
@@ -76,7 +78,8 @@ int launch(const wadg_ctx *c, bool overlap, void (*kern)(KA...), int grid, int t
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = overlap ? 1 : 0;
-  return cuda_check(cudaLaunchKernelEx(&cfg, kern, KA(args)...), "kernel launch");
+  cudaLaunchKernelEx(&cfg, kern, KA(args)...);
+  return after_launch(name);
 }
 
 // CTAs of a persistent kernel over K elements in batches of E: one per batch,
@@ -265,10 +268,9 @@ int launch_vol_pairs_w(const wadg_ctx *c, int K, const double *vgeo, const doubl
     attr.here() = true;
   }
   const int grid = vol_grid<C>(K);
-  if (int r = launch(c, HH > 0 && overlaps<DIM, N>(c, K), kern, grid, C::threads, C::smem_vol, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq,
-                     Dtq, VqLq, VfPq, Qf, rhsQ, rhsQf, c->phys, fgeo, mapPq, blist, nb))
-    return r;
-  return after_launch(SURF ? "volume + surface kernel" : "volume kernel");
+  return launch(c, SURF ? "volume + surface kernel" : "volume kernel", HH > 0 && overlaps<DIM, N>(c, K),
+                kern, grid, C::threads, C::smem_vol, K, vgeo, vfgeo, nrJ, nsJ, ntJ, Drq, Dsq, Dtq, VqLq, VfPq,
+                Qf, rhsQ, rhsQf, c->phys, fgeo, mapPq, blist, nb);
 }
 
 template <int DIM, int N, bool CURVED>
@@ -375,10 +377,8 @@ template <int DIM, int N>
 int launch_surf(const wadg_ctx *c, int K, const double *fgeo, const uint32_t *mapPq,
                 const double *VqLq, const double *Qf, const double *rhsQf, double *rhsQ) {
   using C = SurfMmaCfg<DIM, N>;
-  if (int r = launch(c, overlaps<DIM, N>(c, K), surf_mma_kernel<DIM, N>, (K + C::EW - 1) / C::EW, C::threads, C::smem, K, fgeo,
-                     mapPq, VqLq, Qf, rhsQf, rhsQ, c->phys))
-    return r;
-  return after_launch("surf kernel");
+  return launch(c, "surf kernel", overlaps<DIM, N>(c, K), surf_mma_kernel<DIM, N>, (K + C::EW - 1) / C::EW,
+                C::threads, C::smem, K, fgeo, mapPq, VqLq, Qf, rhsQf, rhsQ, c->phys);
 }
 
 // CTAs of the persistent update kernel: one per group of C::EW elements, at
@@ -450,10 +450,8 @@ int launch_update_w(const wadg_ctx *c, int K, int grid, const double *Jq, const 
                     double *Q, double *Qf, const double *dtK, const int *glist, const int *ng) {
   using C = UpdMmaCfg<DIM, N, CURVED, WIDE>;
   static_assert(C::smem <= 227 * 1024, "update kernel does not fit in shared memory");
-  if (int r = launch(c, overlaps<DIM, N>(c, K), update_mma_kernel<DIM, N, CURVED, WIDE>, grid, C::threads,
-                     C::smem, K, Jq, VqPq, VfPq, fa, fb, fdt, rhsQ, resQ, Q, Qf, c->phys, dtK, glist, ng))
-    return r;
-  return after_launch("update kernel");
+  return launch(c, "update kernel", overlaps<DIM, N>(c, K), update_mma_kernel<DIM, N, CURVED, WIDE>, grid,
+                C::threads, C::smem, K, Jq, VqPq, VfPq, fa, fb, fdt, rhsQ, resQ, Q, Qf, c->phys, dtK, glist, ng);
 }
 
 template <int DIM, int N, bool CURVED>

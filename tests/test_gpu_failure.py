@@ -11,8 +11,9 @@ import numpy as np
 import pytest
 import torch
 
-from scratch_wadge_b200 import capi
+from scratch_wadge_b200 import capi, ic as IC
 from tests.helpers import Case
+from tests.test_gpu_parity import Dev
 
 pytestmark = pytest.mark.gpu
 
@@ -71,3 +72,31 @@ def test_app_check_and_time_loop_stops_on_bad_state(cuda):
     assert ei.value.code == capi.ERR_STATE and "after step 1" in str(ei.value)
     app.set_check_every(0)
     app.sync()  # the stream is still usable
+
+
+@pytest.mark.parametrize("kernel", ["vol", "volsurf", "surf", "update"])
+def test_error_of_a_failed_launch_is_not_the_next_calls(cuda, kernel):
+    """A launch that the runtime refuses (the stream's capture was invalidated by
+    a synchronisation, on the host) returns an error; the calls after it, on a
+    stream that works, do not."""
+    from cuda.bindings import runtime as rt
+    c = Case("tg3d_affine_N3")
+    d = Dev(cuda, c.geo, c.curved)
+    s = d.put(c.state())
+    calls = dict(vol=d.vol, volsurf=d.volsurf, surf=d.surf,
+                 update=lambda s: d.update(s, IC.RK4A[1], IC.RK4B[1], c.dt))
+    calls[kernel](s)  # kernel attributes set
+    d.sync()
+    stream = torch.cuda.Stream()
+    mode = rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal
+    assert rt.cudaStreamBeginCapture(stream.cuda_stream, mode)[0] == 0
+    assert rt.cudaStreamSynchronize(stream.cuda_stream)[0] != 0
+    d.ctx.set_stream(stream.cuda_stream)
+    with pytest.raises(capi.WadgError):
+        calls[kernel](s)
+    rt.cudaStreamEndCapture(stream.cuda_stream)
+    rt.cudaGetLastError()
+    d.ctx.set_stream(torch.cuda.current_stream().cuda_stream)
+    for call in calls.values():
+        call(s)
+    d.sync()
