@@ -14,7 +14,6 @@
 namespace wadg_internal {
 void set_error(const std::string &msg);  // wadg_capi.cu
 }
-void wadg_ctx_set_overlap(wadg_ctx *c, bool on);  // wadg_capi.cu
 
 namespace {
 using wadg_internal::RK4A;
@@ -164,9 +163,9 @@ int capture_step(wadg_app *a, double dt) {
   cudaError_t e = cudaStreamBeginCapture(a->stream, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return afail(WADG_ERR_CUDA, "cudaStreamBeginCapture", e);
   int r = WADG_OK;
-  wadg_ctx_set_overlap(a->ctx, true);
+  wadg_internal::set_overlap(a->ctx, true);
   for (int s = 0; s < 5 && r == WADG_OK; ++s) r = stage(a, RK4A[s], RK4B[s], dt);
-  wadg_ctx_set_overlap(a->ctx, false);
+  wadg_internal::set_overlap(a->ctx, false);
   e = cudaStreamEndCapture(a->stream, &g);
   a->cur = p;  // capture does not execute: restore the parity
   if (r) return r;

@@ -100,13 +100,12 @@ int wadg_ctx_sizes(const wadg_ctx *c, int *dim, int *NfqNf) {
   return WADG_OK;
 }
 
-// see wadg_ctx::overlap (the app, while it captures a time step)
-void wadg_ctx_set_overlap(wadg_ctx *c, bool on) { c->overlap = on; }
-
 // the stream a context's kernels run on (used by wadg_noalloc.cu)
 cudaStream_t wadg_ctx_stream(const wadg_ctx *c) { return c ? c->stream : nullptr; }
 
 namespace wadg_internal {
+void set_overlap(wadg_ctx *c, bool on) { c->overlap = on; }
+
 int vol_automatic(const wadg_ctx *ctx, int curved, int K) {
   wadg_ctx plain = *ctx;  // no shape selected
   plain.vol_warps = plain.vol_rows = 0;

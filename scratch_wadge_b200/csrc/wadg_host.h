@@ -60,6 +60,10 @@ int update_list(const wadg_ctx *c, int K, int curved, const double *Jq, const do
                 const double *VfPq, double fa, double fb, const double *dtK, double *rhsQ,
                 double *resQ, double *Q, double *Qf, const int *glist, const int *ng);
 
+// whether kernels may overlap their predecessor's end (the app, while it captures a time
+// step; wadg_capi.cu)
+void set_overlap(wadg_ctx *c, bool on);
+
 // whether the volume kernel's automatic shape for K elements (vol_warps = 0) is none of
 // wadg_vol_shapes (1; wadg_capi.cu)
 int vol_automatic(const wadg_ctx *c, int curved, int K);

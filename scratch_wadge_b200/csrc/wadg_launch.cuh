@@ -449,7 +449,8 @@ int launch_update_w(const wadg_ctx *c, int K, int grid, const double *Jq, const 
                     const double *VfPq, double fa, double fb, double fdt, double *rhsQ, double *resQ,
                     double *Q, double *Qf, const double *dtK, const int *glist, const int *ng) {
   using C = UpdMmaCfg<DIM, N, CURVED, WIDE>;
-  static_assert(C::smem <= 227 * 1024, "update kernel does not fit in shared memory");
+  // (update_grid raises the limit of the default shape's kernel, not of the wide one's)
+  static_assert(C::smem <= (WIDE ? 48 : 227) * 1024, "update kernel does not fit in shared memory");
   return launch(c, "update kernel", overlaps<DIM, N>(c, K), update_mma_kernel<DIM, N, CURVED, WIDE>, grid,
                 C::threads, C::smem, K, Jq, VqPq, VfPq, fa, fb, fdt, rhsQ, resQ, Q, Qf, c->phys, dtK, glist, ng);
 }
