@@ -34,8 +34,9 @@ exchange are scratch_wadge_b200/partition.py (not benchmarked here).
                   the config's 100 time steps, D2H of Q).  Multi-GPU: independent replicas (the path
                   has no data exchange), max time over ranks.
 --impl reference  the reference's own kernels compiled from its OKL sources
-                  (oracle/_ref, OpenMP over all host cores; the C restatement
-                  when oracle/_ref is absent) on the same workload; rank 0 only.
+                  (oracle/_ref, OpenMP over all host cores) on the same
+                  workload; rank 0 only.  Where oracle/_ref is absent there is
+                  no reference to run: the line says "unavailable".
 """
 
 from __future__ import annotations
@@ -182,10 +183,14 @@ def run_reference(args):
     ws, rank, _ = dist_env()
     if rank != 0:
         return
+    _, kind = cpu_impl()
+    if kind != "reference":  # this repository's restatement is not the reference
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's kernels are not built here "
+                          "(oracle/_ref needs its sources)"}), flush=True)
+        return
     os.environ.setdefault("OMP_NUM_THREADS", str(cpu_threads()))
     geo, st0, dt = build_workload()
     dofs = geo.K * geo.ops.Np
-    _, kind = cpu_impl()
     # each step: one full time step of the whole workload (5 stages)
     if args.warmup > 0:
         time_cpu(geo, st0, dt, min(args.warmup, 1))
