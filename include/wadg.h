@@ -60,11 +60,17 @@ int wadg_ctx_create(const wadg_params *p, wadg_ctx **out);
 int wadg_ctx_destroy(wadg_ctx *ctx);
 int wadg_ctx_set_stream(wadg_ctx *ctx, void *stream);
 /* Tiling of the pair volume kernel: warps per CTA (elements per CTA follow
- * from it; results do not depend on it).  wadg_vol_warps_candidates writes
- * the compiled shapes for the context's degree (at most 3; the first is the
- * default) and returns their number; wadg_ctx_set_vol_warps selects one
- * (0 = the default, which on small meshes takes another shape: a warp per face
- * of an element group).  No counterpart in the reference (OCCA's inner-loop
+ * from it; the results of one node-to-thread map do not depend on it).
+ * wadg_vol_warps_candidates writes the shapes to choose from for the
+ * context's degree (at most 3; the first is what most meshes run by default)
+ * and returns their number; wadg_ctx_set_vol_warps selects one (some other
+ * counts that were candidates once are taken too).  0 = the automatic shape,
+ * chosen by the element count: on small meshes none of the numbered ones but a
+ * warp per face of an element group, which sums an element's columns in
+ * another order.  So automatic and numbered shapes, and one element in meshes
+ * of different sizes, agree to rounding there; a caller who needs the same
+ * bits at every size selects a number.  (The surface flux also takes its
+ * log-mean's polynomial by the face points that share a warp.)  No counterpart in the reference (OCCA's inner-loop
  * sizes are fixed defines); wadg_app_autotune picks one by timing. */
 int wadg_vol_warps_candidates(const wadg_ctx *ctx, int curved, int *out);
 int wadg_ctx_set_vol_warps(wadg_ctx *ctx, int curved, int warps);

@@ -107,8 +107,8 @@ int vol_grid(int K) {
 // candidate CTA shapes of the pair volume kernel (warps per CTA; elements per
 // CTA = warps / 2 * 32 / lanes per element): the default, then two and four
 // warps fewer.  In 2D the second is 16 warps where they fit: four fields need
-// fewer registers (128 per thread), and large 2D meshes run fastest at 16,
-// small ones at 8
+// fewer registers (128 per thread).  Which count is fastest goes with the rounds
+// that a mesh's slices make of it (default_warps)
 template <int DIM, int N, bool CURVED>
 constexpr int volpairsW_cand(int i) {
   constexpr int W0 = volpairsW<DIM, N, CURVED>();
@@ -197,8 +197,10 @@ bool small_mesh(const wadg_ctx *c, int K) {
 // registers per thread cost 2 % in longer runs).  10 time steps, ms, 12 -> 16
 // warps, by slices per SM: N=3 (6 groups for 8) 6.9 1.318 -> 1.223, 13.8 2.10 ->
 // 2.02; curved N=3 6.9 1.58 -> 1.44; N=2 13.8 2.31 -> 2.17; curved N=2 6.9 1.70 ->
-// 1.53; curved N=4 (12 groups for 16) 12.2 2.05 -> 1.83, affine N=4 13.8 (not
-// taken) 1.79 -> 1.81; volume + surface kernel, us, N=1 6.5 23.8 -> 19.6, 7.4 24.3 -> 21.4,
+// 1.53; curved N=4 (12 groups for 16) 12.2 2.05 -> 1.83.  Volume + surface kernel alone
+// at N=4, 16 warps' time over 12's by slices per SM: curved 13.0-13.8 1.00-1.02, 15.6
+// 0.91, 25.9-31.6 0.84-1.03; affine (not taken) 12.3 0.93, 13.0-13.8 1.00-1.01, 15.6 0.92,
+// 26-31 1.02-1.05; volume + surface kernel, us, N=1 6.5 23.8 -> 19.6, 7.4 24.3 -> 21.4,
 // 13.0 33.7 -> 30.2.  Curved 3D N=2: eight where twelve save no round (255 registers a
 // thread for 168), us, 12 -> 8 warps, smooth / random states: 3.7 29.5 -> 27.5 / 40.5 ->
 // 38.9; 6.7 48.7 -> 43.9 / 70.0 -> 65.3; 5.1 (a round against two) 34.6, 8 warps 39.1.  Same bits
@@ -438,7 +440,10 @@ int kernel_shape(const wadg_ctx *c, int kernel, int K, int *E, int *grid) {
 // Meshes of few groups take the wide shape: up to one group per SM in 3D, three
 // in 2D.  Update kernel, us, default -> wide, by groups per SM: 3D N=2 0.1 5.5 ->
 // 4.0, 2.6 6.5 -> 7.3; N=3 0.3 6.9 -> 5.4, 1.1 7.9 -> 8.9; curved N=4 0.6 13.8 -> 11.6,
-// 1.7 20.0 -> 21.4; 2D N=3 1.7 4.6 -> 4.2, 2.7 5.0 -> 4.4, 6.9 7.6 -> 7.9
+// 1.7 20.0 -> 21.4; 2D N=3 1.7 4.6 -> 4.2, 2.7 5.0 -> 4.4, 6.9 7.6 -> 7.9.  Between events
+// (some 4 us more), 2D: N=1, 2 no difference up to 9.7; N=3 1.7 9.7 -> 8.6, 3.9 10.2 -> 9.7,
+// 5.2 11.8 -> 12.4; curved N=4 1.0 10.5 -> 9.8, 2.9 11.9 -> 11.9, 5.2 13.9 -> 17.8; 3D N=2 1.7
+// 10.4 -> 9.8 (not taken), 2.6 10.4 -> 12.3
 template <int DIM, int N, bool CURVED>
 bool wide_update(int K) {
   return K <= (DIM == 3 ? 1 : 3) * num_sms() * UpdMmaCfg<DIM, N, CURVED>::EW;

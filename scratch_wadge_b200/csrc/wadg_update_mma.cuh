@@ -59,7 +59,8 @@ struct UpdMmaCfg {
   // products (the output projection's MO m-tiles go round-robin)
   static constexpr int WARPS = WIDE ? MO : MQ < 2 ? 2 : (MQ > 6 ? 6 : MQ);
   // a warp's m-tiles of the output projection share the fragments of its operand
-  // where it has three of them (3D N=2, 3): 0.0537 -> 0.0499 ms at N=3, K=24576;
+  // where it has three of them (3D N=2, 3): launches back to back, 0.0556 -> 0.0530 ms
+  // at N=3, K=24576 (in a time step 0.0592 -> 0.0554), 0.0264 -> 0.0240 at N=2;
   // the shorter or longer cases (2D; 3D N=4 with its 11 k-steps) lose 1-4 %
   static constexpr bool SHARE = DIM == 3 && (N == 2 || N == 3) && !WIDE;
   static constexpr int threads = 32 * WARPS;
