@@ -199,7 +199,8 @@ __device__ __forceinline__ NodeState<DIM> node_state(const double *q, const Phys
   return s;
 }
 
-// sqrt(x) for x >= 0 (0 for x <= 0): one third-order step on the reciprocal
+// sqrt(x) for x >= 1e-300, else 0 (the estimate takes a subnormal x for 0 and
+// returns infinity; a speed below 1e-150 may count as none): one third-order step on the reciprocal
 // square root estimate y0: with s0 = x y0 and e = 1 - s0 y0, sqrt(x) = s0 (1 -
 // e)^(-1/2) = s0 (1 + e/2 + 3 e^2/8) + O(e^3), |e| < 1.9e-6 (measured
 // over [1, 4)): at most 2.2e-16, in five operations.  For the surface kernels'
@@ -210,7 +211,7 @@ __device__ __forceinline__ double fsqrt(double x) {
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   const double s = x * y;
   const double e = fma(-s, y, 1.0);
-  return x > 0.0 ? fma(s * e, fma(e, 0.375, 0.5), s) : 0.0;
+  return x >= 1e-300 ? fma(s * e, fma(e, 0.375, 0.5), s) : 0.0;
 }
 
 // conservative -> entropy variables (Euler3Daffine.okl:73-93 / Euler2D.okl:69-87)

@@ -15,6 +15,7 @@ from scratch_wadge_b200 import ic as IC
 from scratch_wadge_b200 import mesh as M
 from scratch_wadge_b200.adjoint import Adjoint
 from tests.helpers import RTOL, perturbed, rel
+from tests.test_gpu_parity import Dev
 
 pytestmark = pytest.mark.gpu
 
@@ -116,3 +117,38 @@ def test_meshes_smaller_than_one_group(cuda, dim, n, variant):
     for k in ("Q", "rhsQ", "Qf"):
         assert np.isfinite(out[k]).all()
         assert rel(out[k], ref[k]) < RTOL, (k, rel(out[k], ref[k]))
+
+
+@pytest.mark.parametrize("dim,N,curved", [(3, 3, False), (3, 2, True), (2, 3, False)])
+@pytest.mark.parametrize("speed", [1e-160, 3e-155, 1e-149, 1e-100])
+def test_flow_almost_at_rest(cuda, dim, N, curved, speed):
+    """Velocities whose square is subnormal or underflows: the wave speed is the
+    sound speed, as the reference's kernels give it."""
+    mesh = M.periodic_cube(2, warp=M.warp_cube(0.05) if curved else None) if dim == 3 \
+        else M.periodic_square(6, 5)
+    geo = M.build_geometry(mesh, N)
+    rng = np.random.default_rng(3)
+    U0 = np.empty((dim + 2,) + geo.xyzq.transpose(1, 2, 0).shape[1:])
+    U0[0] = 1.0 + 0.1 * rng.standard_normal(U0[0].shape).clip(-2, 2)
+    U0[1:-1] = 0.0
+    U0[-1] = 2.5 * (1.0 + 0.1 * rng.standard_normal(U0[0].shape).clip(-2, 2))
+    _, rhsQ, Qf, _ = IC.stage0(geo, U0)
+    rhsQ[:, 1:-1] = speed * rhsQ[:, :1]
+    Qf[:, 1:-1] = speed * Qf[:, :1]
+    d = Dev(cuda, geo, curved)
+    ref = Port(geo.ops, curved)
+    want = dict(rhsQ=rhsQ.copy(), Qf=Qf.copy(), rhsQf=np.zeros_like(Qf))
+    ref.vol(geo, want["Qf"], want["rhsQ"], want["rhsQf"])
+    ref.surf(geo, want["Qf"], want["rhsQf"], want["rhsQ"])
+    assert np.isfinite(want["rhsQ"]).all()
+    for fused in (False, True):
+        s = d.put(dict(rhsQ=rhsQ, Qf=Qf, rhsQf=np.zeros_like(Qf)))
+        if fused:
+            d.volsurf(s)
+        else:
+            d.vol(s)
+            d.surf(s)
+        d.sync()
+        h = d.get(s)
+        assert np.isfinite(h["rhsQ"]).all(), fused
+        assert rel(h["rhsQ"], want["rhsQ"]) < RTOL, (fused, rel(h["rhsQ"], want["rhsQ"]))
