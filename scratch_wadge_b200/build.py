@@ -11,6 +11,9 @@ ROOT = os.path.dirname(HERE)
 LIB = os.path.join(HERE, "libwadg_b200.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
+# uncompressed device code: nvcc compresses what is over some 10 MB, and a degree's first
+# kernel in a process then takes 8-12 ms to unpack its object instead of 5-6 to load it
+COMPRESS = ["-compress-mode=none"]
 
 
 def sources():
@@ -33,7 +36,7 @@ def build(force=False, verbose=False, extra=()):
     procs = []
     for src in sources():
         obj = os.path.join(bdir, os.path.basename(src) + ".o")
-        cmd = [NVCC, "-O3", "-std=c++17", *ARCH, "-lineinfo", "-Xcompiler", "-fPIC",
+        cmd = [NVCC, "-O3", "-std=c++17", *ARCH, *COMPRESS, "-lineinfo", "-Xcompiler", "-fPIC",
                "-Xptxas", "-v" if verbose else "-O3", "-I", os.path.join(ROOT, "include"),
                "-c", src, "-o", obj, *extra]
         procs.append((cmd, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
